@@ -26,6 +26,9 @@ namespace
 {
 using namespace lv;
 
+/* the voxel types other than uint8 and uint16, a run-time switch */
+constexpr int kDtAny = -1;
+
 struct HistJob
 {
     uint64_t offset; /* brick byte offset in the pool */

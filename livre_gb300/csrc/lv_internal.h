@@ -78,11 +78,6 @@ struct LodView
     uint32_t* result;     /* LV_SELECT_RESULT_WORDS */
 };
 
-/* Voxel-type template argument of the ray-cast kernels for the types other
- * than uint8 and uint16 (int8, int16, uint32, int32, float), read through a
- * run-time switch on RayView::dtype. */
-constexpr int kDtAny = -1;
-
 /* Per-view constants of the ray cast. */
 struct RayView
 {

@@ -390,6 +390,10 @@ void batch_decode_stats(const uint32_t* words, lv_frame_stats& s);
 lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
                               uint8_t* order_scratch, cudaStream_t s);
 size_t tile_order_bytes(const RayView& V, const lv_render_launch& L);
+/* The ray cast of a voxel type other than uint8 and uint16 (raycast_types.cu):
+ * one CTA per tile of L, block i on tile order[i] (null: tile i). */
+lv_status launch_other_type(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
+                            const uint32_t* order, cudaStream_t s);
 /* Longest-first order of a batched group's work items (memset + 2 kernels);
  * hist: 128 words, keys and order: max_items entries (an upper bound of the
  * group's items at every replay of a captured launch). */
