@@ -87,6 +87,13 @@ struct RayView
     float nearp;
     float gmin[3], gmax[3], gscale[3];
     float goff[3];    /* half world size * gscale: f = fma(p, gscale, goff) */
+    /* constants of the brick lookup (locate), per axis: the eye's cell
+     * coordinate fma(eye, gscale, goff); the clamp of a sample's cell
+     * coordinate that makes one past the high face the face cell (dims - 1/2
+     * on the axes with the most cells, out of reach on the others); where the
+     * last cell ends for a sample (infinity or dims); block size; overlap
+     * minus the half texel of the filter */
+    float f0[3], cell_hi[3], cube_end[3], Bf[3], Oh[3];
     float clip[6][4];
     uint32_t n_clip;
     uint32_t dims[3]; /* leaf grid (finest level) */

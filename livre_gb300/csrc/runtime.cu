@@ -864,6 +864,11 @@ lv_status make_ray_view(lv_ctx* ctx, const lv_volume* vol, const lv_tf* tf,
         V.N[a] = info.max_block[a];
         V.O[a] = info.overlap[a];
         V.B[a] = info.max_block[a] - 2u * info.overlap[a];
+        V.f0[a] = std::fma(V.eye[a], V.gscale[a], V.goff[a]);
+        V.cell_hi[a] = dims[a] == bm ? float(dims[a]) - 0.5f : 4194304.0f;
+        V.cube_end[a] = dims[a] == bm ? std::numeric_limits<float>::infinity() : float(dims[a]);
+        V.Bf[a] = float(V.B[a]);
+        V.Oh[a] = float(V.O[a]) - (desc.filter == LV_FILTER_TRILINEAR ? 0.5f : 0.0f);
         if (info.overlap[a] == 0 || V.N[a] < 2)
             V.edge = 1;
     }
