@@ -451,7 +451,9 @@ lv_status prepare_view_kernels(lv_batch* b, uint32_t n)
     b->view_offs.assign(n + 1, 0);
     for (uint32_t i = 0; i < n; ++i)
         b->view_offs[i + 1] =
-            b->view_offs[i] + ((tile_order_bytes(h_rays[i], L) + 255) & ~size_t(255));
+            b->view_offs[i] +
+            ((tile_order_bytes(h_rays[i], ray_launch(h_rays[i], L, ~uint64_t(0))) + 255) &
+             ~size_t(255));
     if (b->cfg.order == LV_ORDER_LONGEST_FIRST && b->view_scratch.bytes < b->view_offs[n])
     {
         LV_CUDA(ctx, cudaStreamSynchronize(b->stream));
@@ -618,7 +620,8 @@ lv_status enqueue_batch(lv_batch* b, uint32_t n, const std::vector<Group>& group
                                    ? b->view_scratch.as<uint8_t>() + offs[i]
                                    : nullptr;
             cudaStream_t vs = aux[j % n_streams];
-            st = launch_view_raycast(ctx, h_rays[i], L, scratch, vs);
+            st = launch_view_raycast(ctx, h_rays[i], ray_launch(h_rays[i], L, ~uint64_t(0)), scratch,
+                                     vs);
             if (st != LV_OK)
                 return st;
             if (b->hook)

@@ -206,9 +206,19 @@ lv_status run_selection(lv_ctx* ctx, const LodView* host_views,
                         uint32_t n_views, uint32_t max_depth,
                         cudaStream_t stream, bool allow_fused = true);
 
-/* The launch the ray cast of V really uses under L (other voxel types than
- * uint8 / uint16 always use one CTA per tile). */
-lv_render_launch effective_launch(const RayView& V, const lv_render_launch& L);
+/* The ray cast of a view as launched: its shape and the lanes that share a
+ * ray (1, or 4 or 8 with one CTA per tile). */
+struct RayLaunch
+{
+    lv_render_launch shape;
+    uint32_t lanes;
+};
+/* Pixels of V whose ray can reach the volume (its screen rectangle within
+ * the rendered rect). */
+uint64_t candidate_rays(const RayView& V);
+/* The launch the ray cast of V uses under L when `rays` candidate rays are
+ * cast at once (V's own, or those of all views of a batch). */
+RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays);
 /* lv_render's tile order for V under L, computed on `side` into the
  * renderer's tile scratch (null for raster order or the per-pixel grid). */
 lv_status prepare_frame_order(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
@@ -384,16 +394,19 @@ void batch_set_priority_level(lv_batch* b, int level);
 /* Frame statistics from a view's counter words. */
 void batch_decode_stats(const uint32_t* words, lv_frame_stats& s);
 
-/* One view's ray cast with launch shape L, its longest-first tile order (if
- * any) in `order_scratch` (tile_order_bytes; nullptr: the context's lv_render
+/* One view's ray cast as launch R, its longest-first tile order (if any) in `order_scratch` (tile_order_bytes; nullptr: the context's lv_render
  * scratch). The view's samples per ray must already be in its counters. */
-lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
+lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const RayLaunch& R,
                               uint8_t* order_scratch, cudaStream_t s);
-size_t tile_order_bytes(const RayView& V, const lv_render_launch& L);
-/* The ray cast of a voxel type other than uint8 and uint16 (raycast_types.cu):
- * one CTA per tile of L, block i on tile order[i] (null: tile i). */
+size_t tile_order_bytes(const RayView& V, const RayLaunch& R);
+/* The ray cast of a voxel type other than uint8 and uint16 (raycast_types.cu),
+ * and of uint8 and uint16 with 4 or 8 lanes per ray (raycast_split.cu, `pitch`
+ * the fixed pitch or 0): one CTA per tile of L, block i on tile order[i]
+ * (null: tile i). */
 lv_status launch_other_type(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
-                            const uint32_t* order, cudaStream_t s);
+                            uint32_t lanes, const uint32_t* order, cudaStream_t s);
+lv_status launch_split(lv_ctx* ctx, const RayView& V, const lv_render_launch& L, uint32_t lanes,
+                       uint32_t pitch, const uint32_t* order, cudaStream_t s);
 /* Longest-first order of a batched group's work items (memset + 2 kernels);
  * hist: 128 words, keys and order: max_items entries (an upper bound of the
  * group's items at every replay of a captured launch). */

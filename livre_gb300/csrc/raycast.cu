@@ -26,7 +26,8 @@
  *
  * raycast_device.cuh holds the device code of a ray; this file the residency
  * and leaf-grid kernels, the launches of uint8 and uint16 volumes and the
- * dispatch; raycast_types.cu the launches of the other voxel types.
+ * dispatch; raycast_split.cu those with several lanes per ray and
+ * raycast_types.cu the launches of the other voxel types.
  */
 #include <algorithm>
 #include <cmath>
@@ -979,26 +980,83 @@ uint8_t* render_order_scratch(lv_ctx* ctx, const RayView& V, const lv_render_lau
 
 } // namespace
 
-lv_render_launch effective_launch(const RayView& V, const lv_render_launch& L)
+uint64_t candidate_rays(const RayView& V)
 {
-    if (V.dtype == LV_DT_UINT8 || V.dtype == LV_DT_UINT16)
-        return L;
-    lv_render_launch T = L;
-    T.kind = LV_LAUNCH_TILE_GRID;
-    const uint32_t px = T.tile_w * T.tile_h;
-    if (px == 0 || px > 256 || px % 32 != 0)
+    const uint32_t x0 = std::max(V.x0, V.cull[0]), x1 = std::min(V.x0 + V.W, V.cull[2]);
+    const uint32_t y0 = std::max(V.y0, V.cull[1]), y1 = std::min(V.y0 + V.H, V.cull[3]);
+    return x0 < x1 && y0 < y1 ? uint64_t(x1 - x0) * (y1 - y0) : 0;
+}
+
+namespace
+{
+/* The fixed pitch whose kernels render V (34, 66, 130: the 32^3, 64^3 and
+ * 128^3 bricks with an overlap of 1), or 0. */
+uint32_t fixed_pitch(const RayView& V)
+{
+    const bool fixed = V.edge == 0 && V.filter == LV_FILTER_TRILINEAR && V.N[0] == V.N[1] &&
+                       (V.N[0] == 34 || V.N[0] == 66 || V.N[0] == 130) && fixed_pitch_layout(V);
+    return fixed ? V.N[0] : 0;
+}
+
+/* Lanes that share a ray in a launch of `rays` candidate rays (pixels that
+ * can reach the volume) under the default launch; other launch shapes keep
+ * one lane per ray. Few rays leave most of the 152 SMs' issue slots idle
+ * behind chains of dependent loads, so their samples go to more lanes; the
+ * exchange costs instructions, which a frame that fills the GPU pays for.
+ * Ray-cast us with 1 / 4 / 8 lanes, orbits at 1.6 volume diagonals:
+ *                        2 255 rays    29 575       114 208        394 885
+ *   uint8 64^3, 1 px     41  18  14    174  69  85   518 392 434   1029 1082
+ *   uint8 64^3, 2 px     41  18  14     76  43  57   188 208 243    939 1069
+ *   uint8 32^3           49  20  17    164  69  86   217 186 227    393  505
+ *   uint16 64^3          44  19  16    173  80 109   921 527 543   2188 1468
+ *   uint16 128^3, 2 px  108  41  34    119  61  73   245 202 233    733  716
+ *   float 48^3          397 113  53    501 153 108   543 279 320    980  734
+ *   int16 64^3          358 102  51    404 150 143   555 405 429   1290  965
+ *   uint8 nearest       184  61  37    393 117 104   344 235 270    638  589
+ *   uint8 clamped       258  57  35    379 120 110   839 338 320   1135  735
+ * The trilinear uint8 kernels have the fewest loads per sample, so they fill
+ * the issue slots with the fewest rays; types with eight loads or with
+ * clamped taps gain from the shared cache lines to 400 000 rays and (float,
+ * int16, uint16 64^3) beyond, where uint16 128^3 and the nearest filter
+ * lose. */
+uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
+{
+    if (L.kind != LV_LAUNCH_TILE_GRID || L.tile_w != 8 || L.tile_h != 8 || !L.lookahead)
+        return 1;
+    const bool light = V.dtype == LV_DT_UINT8 && V.filter == LV_FILTER_TRILINEAR && !V.edge;
+    const uint64_t eight = light ? 8192 : V.dtype == LV_DT_UINT16 ? 16384 : 32768;
+    const uint64_t four = light ? 81920 : 409600;
+    return rays <= eight ? 8 : rays <= four ? 4 : 1;
+}
+} // namespace
+
+RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays)
+{
+    RayLaunch R{L, split_lanes(V, L, rays)};
+    if (R.lanes > 1)
     {
-        T.tile_w = 8;
-        T.tile_h = 16;
+        /* 64 threads: 4 x 4 pixels of 4 lanes or 4 x 2 of 8 */
+        R.shape.tile_w = 4;
+        R.shape.tile_h = 16 / R.lanes;
     }
-    return T;
+    else if (V.dtype != LV_DT_UINT8 && V.dtype != LV_DT_UINT16)
+    {
+        R.shape.kind = LV_LAUNCH_TILE_GRID;
+        const uint32_t px = L.tile_w * L.tile_h;
+        if (px == 0 || px > 256 || px % 32 != 0)
+        {
+            R.shape.tile_w = 8;
+            R.shape.tile_h = 16;
+        }
+    }
+    return R;
 }
 
 lv_status prepare_frame_order(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
                               cudaStream_t side, const uint32_t*& order)
 {
     order = nullptr;
-    const lv_render_launch T = effective_launch(V, L);
+    const lv_render_launch T = ray_launch(V, L, candidate_rays(V)).shape;
     if (T.kind == LV_LAUNCH_GRID || T.order != LV_ORDER_LONGEST_FIRST)
         return LV_OK;
     lv_status st = LV_OK;
@@ -1127,9 +1185,7 @@ template <int DT, int F, int EDGE>
 lv_status plain_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
                          cudaStream_t s, uint8_t* scratch)
 {
-    if (EDGE == 0 && F == LV_FILTER_TRILINEAR && L.kind == LV_LAUNCH_TILE_GRID &&
-        V.N[0] == V.N[1] && (V.N[0] == 66 || V.N[0] == 34 || V.N[0] == 130) &&
-        fixed_pitch_layout(V))
+    if (EDGE == 0 && F == LV_FILTER_TRILINEAR && L.kind == LV_LAUNCH_TILE_GRID && fixed_pitch(V))
     {
         if (L.lookahead)
             return V.N[0] == 66   ? tiles_nx_dispatch<DT, F, 66, 1>(ctx, V, L, s, scratch)
@@ -1193,21 +1249,18 @@ lv_status refill_views_by_index(int idx, lv_ctx* ctx, const RayView* d, const Ti
 }
 } // namespace
 
-size_t tile_order_bytes(const RayView& V, const lv_render_launch& L)
+size_t tile_order_bytes(const RayView& V, const RayLaunch& R)
 {
-    return order_bytes_of(V, L);
+    return order_bytes_of(V, R.shape);
 }
 
 int batch_group(const RayView& V)
 {
     const int v = kernel_variant(V.dtype, V.filter, V.edge);
-    if (v >= 8 || V.filter != LV_FILTER_TRILINEAR || V.edge != 0 || V.N[0] != V.N[1] ||
-        !fixed_pitch_layout(V))
+    const uint32_t pitch = fixed_pitch(V);
+    if (v >= 8 || pitch == 0)
         return v < 8 ? v : kBatchGroups + v;
-    const int pitch = V.N[0] == 34 ? 0 : V.N[0] == 66 ? 1 : V.N[0] == 130 ? 2 : -1;
-    if (pitch < 0)
-        return v;
-    return 8 + (V.dtype == LV_DT_UINT16 ? 3 : 0) + pitch;
+    return 8 + (V.dtype == LV_DT_UINT16 ? 3 : 0) + (pitch == 34 ? 0 : pitch == 66 ? 1 : 2);
 }
 
 /* 0..7: uint8 / uint16 x filter x edge; 8..11: the other voxel types x
@@ -1220,37 +1273,31 @@ int kernel_variant(uint32_t dtype, uint32_t filter, uint32_t edge)
     return (dtype == LV_DT_UINT16 ? 4 : 0) + fe;
 }
 
-/* The voxel types other than uint8 / uint16 always use one CTA per tile,
- * with the launch's tile shape (8 x 16 when it is not a CTA's), order and
- * look-ahead. */
-static lv_status other_type_raycast(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
-                                    cudaStream_t s, uint8_t* scratch)
-{
-    const lv_render_launch T = effective_launch(V, L);
-    lv_status st = LV_OK;
-    const uint32_t* order = frame_order(ctx, V, T, scratch, s, st);
-    if (st != LV_OK)
-        return st;
-    return launch_other_type(ctx, V, T, order, s);
-}
-
 lv_status launch_raycast(lv_ctx* ctx, const RayView& V, cudaStream_t s)
 {
     if (V.dtype > LV_DT_INT32)
         return fail(ctx, LV_EINVAL, "unknown voxel type");
     /* the ray-cast kernels derive the samples per ray themselves */
-    return launch_view_raycast(ctx, V, ctx->launch, nullptr, s);
+    return launch_view_raycast(ctx, V, ray_launch(V, ctx->launch, candidate_rays(V)), nullptr, s);
 }
 
-lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
+lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const RayLaunch& R,
                               uint8_t* order_scratch, cudaStream_t s)
 {
+    const lv_render_launch& L = R.shape;
+    const bool other = V.dtype != LV_DT_UINT8 && V.dtype != LV_DT_UINT16;
+    if (other || R.lanes > 1)
+    {
+        /* one CTA per tile */
+        lv_status st = LV_OK;
+        const uint32_t* order = frame_order(ctx, V, L, order_scratch, s, st);
+        if (st != LV_OK)
+            return st;
+        return other ? launch_other_type(ctx, V, L, R.lanes, order, s)
+                     : launch_split(ctx, V, L, R.lanes, fixed_pitch(V), order, s);
+    }
     switch (kernel_variant(V.dtype, V.filter, V.edge))
     {
-    case 8:
-    case 9:
-    case 10:
-    case 11: return other_type_raycast(ctx, V, L, s, order_scratch);
     case 0: return plain_dispatch<LV_DT_UINT8, 0, 0>(ctx, V, L, s, order_scratch);
     case 1: return plain_dispatch<LV_DT_UINT8, 0, 1>(ctx, V, L, s, order_scratch);
     case 2: return plain_dispatch<LV_DT_UINT8, 1, 0>(ctx, V, L, s, order_scratch);

@@ -626,13 +626,13 @@ __device__ __forceinline__ bool locate(const RayView& V, RayState& r, float step
     return true;
 }
 
-/* Advances the ray to its next sample (index r.kf) with one divergent
+/* Takes the ray's sample r.kf and advances it by STRIDE samples, with one divergent
  * region, the brick lookup where the ray leaves its safe range; false once
  * the ray has left its segment. The sample's voxels are read into T only
  * when it has data (`valid`: inside the segment and in a rendered brick, not
  * outside the octree or in a cell no brick covers), by predicated loads, so
  * a sample without data costs no branch. */
-template <int DT, int FILTER, int EDGE, class HV>
+template <int DT, int FILTER, int EDGE, int STRIDE = 1, class HV>
 __device__ __forceinline__ bool fetch_sample(const RayView& V, const HV& H, RayState& r, float step,
                                          Taps<FILTER>& T, bool& valid)
 {
@@ -645,7 +645,7 @@ __device__ __forceinline__ bool fetch_sample(const RayView& V, const HV& H, RayS
         if (!locate<FILTER>(V, r, step, f))
             r.entry = kLeafEmpty; /* outside the octree: this sample has no data */
     }
-    r.kf += 1.0f;
+    r.kf += float(STRIDE);
     valid = live && r.entry != kLeafEmpty;
     float sc[3];
 #pragma unroll
@@ -786,5 +786,200 @@ __global__ void __launch_bounds__(256)
     if ((threadIdx.x & 31u) == 0 && sum)
         atomicAdd(reinterpret_cast<unsigned long long*>(V.counters + FC_SAMPLES_LO), sum);
 }
+
+/* ---------------------------------------------------------- split rays
+ * S lanes of a warp share a ray: lane j takes its samples j, j + S, j + 2S,
+ * ... In each iteration they fetch, interpolate and classify S consecutive
+ * samples side by side and exchange the colours and opacities through shared
+ * memory; lane j then blends channel j % 4 of all S, in sample order. So the
+ * samples, their values, the blending order and the roundings are march()'s
+ * (image and sample count bit for bit), while a ray's chain of dependent
+ * loads is S times shorter, a frame has S times more warps, and the lanes of
+ * a warp read S consecutive positions of 32 / S rays instead of one position
+ * of 32 rays, which touches fewer cache lines where a pixel spans a voxel or
+ * more (uint8 quads, one voxel per pixel, S = 4: 3.4 L1 wavefronts per load
+ * request against 6.6).
+ *
+ * The price is the exchange and S blends instead of one, about 60
+ * instructions on 85 with S = 4, so a frame of many rays whose issue slots
+ * are busy is faster with one lane per ray: split_lanes (raycast.cu) chooses. */
+template <int S>
+struct RayGroup
+{
+    /* a ray's row of the exchange buffer: 4 planes (red, green, blue,
+     * opacity) of S values, padded so that a warp's plane write (32 / S rows)
+     * hits 32 banks */
+    static constexpr int kRow = S == 4 ? 20 : 4 * S + 8;
+    float c; /* this lane's channel, blended so far (lanes 3 mod 4: blue again) */
+    float a; /* the opacity, in every lane */
+
+    __device__ __forceinline__ static uint32_t plane(uint32_t j) { return min(j & 3u, 2u) * S; }
+
+    __device__ __forceinline__ void blend(float v, float alpha)
+    {
+        /* composite_sample's blend */
+        const float w = alpha * (1.0f - a);
+        c = fmaf(v, w, c);
+        a = fmaf(alpha, 1.0f - a, a);
+    }
+
+    /* blends a row; true, with the group as before, when the opacity passed
+     * `early` on the way */
+    __device__ __forceinline__ bool blend_row(const float* row, uint32_t j, float early)
+    {
+        const RayGroup was = *this;
+        bool stop = false;
+#pragma unroll
+        for (int q = 0; q < S; q += 4)
+        {
+            const float4 alpha = *reinterpret_cast<const float4*>(row + 3 * S + q);
+            const float4 v = *reinterpret_cast<const float4*>(row + plane(j) + q);
+            blend(v.x, alpha.x);
+            stop = stop || a > early;
+            blend(v.y, alpha.y);
+            stop = stop || a > early;
+            blend(v.z, alpha.z);
+            stop = stop || a > early;
+            blend(v.w, alpha.w);
+            stop = stop || a > early;
+        }
+        if (stop)
+            *this = was;
+        return stop;
+    }
+
+    /* blends a row up to and with the sample that passes `early` and returns
+     * that sample's place (the last place if none does) */
+    __device__ __forceinline__ uint32_t blend_to_stop(const float* row, uint32_t j, float early)
+    {
+        for (uint32_t i = 0;; ++i)
+        {
+            blend(row[plane(j) + i], row[3 * S + i]);
+            if (a > early || i == uint32_t(S) - 1u)
+                return i;
+        }
+    }
+};
+
+/* The colour of one sample and its opacity corrected for the step (the first
+ * half of composite_sample); all 0 when the sample has no data, so that
+ * whatever its unread voxels map to (an infinite table entry, say) leaves the
+ * ray as it is. */
+template <int FILTER, bool RAW, class HV>
+__device__ __forceinline__ float4 classify_sample(const HV& H, float ac, const Taps<FILTER>& T,
+                                                  bool valid)
+{
+    float4 src = tf_lookup<0>(H, interp<FILTER, RAW>(T));
+    const float am = fminf(src.w, 1.0f - 1.0f / 256.0f);
+    src.w = 1.0f - ex2_approx(ac * lg2_approx(1.0f - am));
+    return valid ? src : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+constexpr uint32_t kSplitThreads = 64;
+constexpr float kRayOver = -3.0e38f; /* RayState::thi of a ray with no sample left */
+
+/* One CTA of kSplitThreads threads per tile of tile_w * tile_h =
+ * kSplitThreads / S pixels, S lanes to a ray; block i renders tile order[i]
+ * (null: tile i). One sample of look-ahead per lane, as march(). */
+template <int DT, int FILTER, int EDGE, int S>
+__global__ void __launch_bounds__(kSplitThreads)
+    raycast_split_kernel(const RayView V, uint32_t tile_w, uint32_t tile_h,
+                         const uint32_t* __restrict__ order)
+{
+    if (skip_frame(V))
+        return;
+    /* two rows per ray in turn: by the time a lane writes a row again, every
+     * lane has read it, since all have passed the other row's barrier */
+    __shared__ alignas(16) float rows[2][kSplitThreads / S * RayGroup<S>::kRow];
+    constexpr bool RAW = raw_taps<DT, FILTER, EDGE>();
+    const uint32_t n = frame_samples(V);
+    const float step = __fdiv_rn(1.0f, __uint2float_rn(n));
+    const float ac = __fdiv_rn(32.0f, __uint2float_rn(n));
+    const uint32_t tiles_x = (V.W + tile_w - 1) / tile_w;
+    const uint32_t tile = order ? order[blockIdx.x] : blockIdx.x;
+    const uint32_t ray = threadIdx.x / S, j = threadIdx.x % S;
+    const uint32_t px = (tile % tiles_x) * tile_w + ray % tile_w;
+    const uint32_t py = (tile / tiles_x) * tile_h + ray / tile_w;
+    const bool in = px < V.W && py < V.H;
+    RayGeom g;
+    g.dir[0] = g.dir[1] = g.dir[2] = g.tg = g.tlo = g.thi = 0.0f;
+    g.hit = false;
+    float4 init = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (in)
+    {
+        g = ray_setup(V, px, py);
+        init = initial_dst(V, px, py);
+    }
+    RayState r;
+    r.tg = r.kf = 0.0f;
+    r.kf_safe = -1.0f;
+    r.err = 0u;
+    r.entry = kLeafEmpty;
+    r.brick = nullptr;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        r.dir[a] = r.sa[a] = r.sb[a] = 0.0f;
+    if (!ray_begin(g, step, r) || init.w > V.early)
+        r.thi = kRayOver;
+    r.kf += float(j);
+    RayGroup<S> G;
+    G.c = (j & 3u) == 0u ? init.x : (j & 3u) == 1u ? init.y : init.z;
+    G.a = init.w;
+    float* row0 = rows[0] + ray * RayGroup<S>::kRow;
+    float* row1 = rows[1] + ray * RayGroup<S>::kRow;
+    uint32_t nsamp = 0;
+    auto composite = [&](float* row, const Taps<FILTER>& T, bool valid) {
+        const float4 src = classify_sample<FILTER, RAW>(V, ac, T, valid);
+        row[j] = src.x;
+        row[S + j] = src.y;
+        row[2 * S + j] = src.z;
+        row[3 * S + j] = src.w;
+        __syncwarp();
+        nsamp += valid ? 1u : 0u;
+        if (G.blend_row(row, j, V.early) && r.thi != kRayOver)
+        {
+            /* the ray ends within this row (once per ray): the samples after
+             * the one that passed the opacity do not count */
+            const uint32_t last = G.blend_to_stop(row, j, V.early);
+            if (valid && j > last)
+                --nsamp;
+            r.thi = kRayOver;
+        }
+    };
+    Taps<FILTER> T0, T1;
+    bool v0, v1;
+    bool live = fetch_sample<DT, FILTER, EDGE, S>(V, V, r, step, T0, v0);
+    while (__any_sync(0xFFFFFFFFu, live))
+    {
+        fetch_sample<DT, FILTER, EDGE, S>(V, V, r, step, T1, v1);
+        composite(row0, T0, v0);
+        v1 = v1 && r.thi != kRayOver;
+        live = fetch_sample<DT, FILTER, EDGE, S>(V, V, r, step, T0, v0);
+        composite(row1, T1, v1);
+        v0 = v0 && r.thi != kRayOver;
+    }
+    flush_error(V, r);
+    if (in && j < 4u)
+        reinterpret_cast<float*>(V.out + frame_index(V, px, py))[j] = j == 3u ? G.a : G.c;
+    unsigned long long sum = nsamp;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        sum += __shfl_down_sync(0xFFFFFFFFu, sum, o);
+    if ((threadIdx.x & 31u) == 0 && sum)
+        atomicAdd(reinterpret_cast<unsigned long long*>(V.counters + FC_SAMPLES_LO), sum);
+}
+
+template <int DT, int FILTER, int EDGE>
+lv_status split_launch(lv_ctx* ctx, const RayView& V, const lv_render_launch& L, uint32_t lanes,
+                       const uint32_t* order, cudaStream_t s)
+{
+    const uint32_t tiles = ((V.W + L.tile_w - 1) / L.tile_w) * ((V.H + L.tile_h - 1) / L.tile_h);
+    auto k = lanes == 4 ? raycast_split_kernel<DT, FILTER, EDGE, 4>
+                        : raycast_split_kernel<DT, FILTER, EDGE, 8>;
+    k<<<tiles, kSplitThreads, 0, s>>>(V, L.tile_w, L.tile_h, order);
+    LV_CUDA(ctx, cudaGetLastError());
+    return LV_OK;
+}
+
 } // namespace
 } // namespace lv
