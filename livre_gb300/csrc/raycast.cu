@@ -813,6 +813,22 @@ __global__ void __launch_bounds__(kRefillThreads, kRefillMinCtas)
         atomicMax(Q.clock + 1, globaltimer());
 }
 
+/* Transparent black in the pixels of V's rect that lie outside
+ * [ix0, ix1) x [iy0, iy1). */
+__global__ void __launch_bounds__(256)
+    clear_outside_kernel(float4* __restrict__ out, uint32_t FW, uint32_t x0, uint32_t y0,
+                         uint32_t W, uint32_t H, uint32_t ix0, uint32_t iy0, uint32_t ix1,
+                         uint32_t iy1)
+{
+    const uint32_t x = x0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= x0 + W)
+        return;
+    const bool column = x >= ix0 && x < ix1;
+    for (uint32_t y = y0 + blockIdx.y; y < y0 + H; y += gridDim.y)
+        if (!(column && y >= iy0 && y < iy1))
+            out[uint64_t(y) * FW + x] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 __global__ void to_rgba8_kernel(const float4* __restrict__ in,
                                 uchar4* __restrict__ out, uint64_t n)
 {
@@ -979,6 +995,32 @@ uint8_t* render_order_scratch(lv_ctx* ctx, const RayView& V, const lv_render_lau
 }
 
 } // namespace
+
+lv_status shrink_to_candidates(lv_ctx* ctx, RayView& V, cudaStream_t s)
+{
+    /* corners on multiples of 8 pixels: a row of a tile is a whole 128-byte
+     * line of the frame */
+    uint32_t x0 = std::max(V.x0, V.cull[0] & ~7u), x1 = std::min(V.x0 + V.W, V.cull[2]);
+    uint32_t y0 = std::max(V.y0, V.cull[1] & ~7u), y1 = std::min(V.y0 + V.H, V.cull[3]);
+    if (x0 >= x1 || y0 >= y1)
+    {
+        /* nothing to see: one pixel, for the launch to report the frame */
+        x0 = V.x0;
+        y0 = V.y0;
+        x1 = x0 + 1;
+        y1 = y0 + 1;
+    }
+    if (uint64_t(x1 - x0) * (y1 - y0) == uint64_t(V.W) * V.H)
+        return LV_OK;
+    clear_outside_kernel<<<dim3((V.W + 255) / 256, std::min(V.H, 2048u)), 256, 0, s>>>(
+        V.out, V.FW, V.x0, V.y0, V.W, V.H, x0, y0, x1, y1);
+    LV_CUDA(ctx, cudaGetLastError());
+    V.x0 = x0;
+    V.y0 = y0;
+    V.W = x1 - x0;
+    V.H = y1 - y0;
+    return LV_OK;
+}
 
 uint64_t candidate_rays(const RayView& V)
 {

@@ -1650,10 +1650,14 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
                        R.counters.as<uint32_t>(), V);
     if (st != LV_OK)
         return st;
-    /* from the camera alone, beside the selection: the longest-first tile
-     * order and the cleared leaf grid; the leaf fill waits for both */
+    /* from the camera alone, beside the selection: the cleared leaf grid, the
+     * pixels no ray of which can reach the volume and the longest-first tile
+     * order of the others; the leaf fill waits for them */
     LV_CUDA(ctx, cudaStreamWaitEvent(R.side, R.fork, 0));
     LV_CUDA(ctx, cudaMemsetAsync(R.leaf.ptr, 0xFF, cells * sizeof(uint32_t), R.side));
+    st = shrink_to_candidates(ctx, V, R.side);
+    if (st != LV_OK)
+        return st;
     st = prepare_frame_order(ctx, V, ctx->launch, R.side, R.pre_order);
     if (st != LV_OK)
         return st;
