@@ -77,6 +77,7 @@ struct lv_batch
      * and ray-cast timing */
     lv::DeviceBuffer view_scratch;
     std::vector<uint64_t> view_offs;
+    uint64_t rays = 0; /* candidate rays of all views */
     cudaEvent_t t_vk0 = nullptr, t_vk1 = nullptr;
     bool vk_timed = false;
     /* per-view completion hook (per-view kernels only) */
@@ -448,11 +449,14 @@ lv_status prepare_view_kernels(lv_batch* b, uint32_t n)
     const RayView* h_rays = reinterpret_cast<const RayView*>(b->h_params.as<uint8_t>() + PL.ray);
     const lv_render_launch L{LV_LAUNCH_TILE_GRID, b->cfg.tile_w, b->cfg.tile_h, 0,
                              b->cfg.order, b->cfg.lookahead};
+    b->rays = 0;
+    for (uint32_t i = 0; i < n; ++i)
+        b->rays += candidate_rays(h_rays[i]);
     b->view_offs.assign(n + 1, 0);
     for (uint32_t i = 0; i < n; ++i)
         b->view_offs[i + 1] =
             b->view_offs[i] +
-            ((tile_order_bytes(h_rays[i], ray_launch(h_rays[i], L, ~uint64_t(0))) + 255) &
+            ((tile_order_bytes(h_rays[i], ray_launch(h_rays[i], L, b->rays)) + 255) &
              ~size_t(255));
     if (b->cfg.order == LV_ORDER_LONGEST_FIRST && b->view_scratch.bytes < b->view_offs[n])
     {
@@ -620,8 +624,7 @@ lv_status enqueue_batch(lv_batch* b, uint32_t n, const std::vector<Group>& group
                                    ? b->view_scratch.as<uint8_t>() + offs[i]
                                    : nullptr;
             cudaStream_t vs = aux[j % n_streams];
-            st = launch_view_raycast(ctx, h_rays[i], ray_launch(h_rays[i], L, ~uint64_t(0)), scratch,
-                                     vs);
+            st = launch_view_raycast(ctx, h_rays[i], ray_launch(h_rays[i], L, b->rays), scratch, vs);
             if (st != LV_OK)
                 return st;
             if (b->hook)

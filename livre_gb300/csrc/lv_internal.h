@@ -125,6 +125,7 @@ struct RayView
                                a conservative bound of the pixels whose ray can
                                reach the volume's box; the others start and end
                                with no sample */
+    float px_per_voxel;     /* estimated screen size of a rendered voxel's side */
     uint32_t samples_fixed; /* 0 = policy */
     uint32_t step_policy;
     uint32_t max_voxel_dim;

@@ -1044,30 +1044,46 @@ uint32_t fixed_pitch(const RayView& V)
  * can reach the volume) under the default launch; other launch shapes keep
  * one lane per ray. Few rays leave most of the 152 SMs' issue slots idle
  * behind chains of dependent loads, so their samples go to more lanes; the
- * exchange costs instructions, which a frame that fills the GPU pays for.
- * Ray-cast us with 1 / 4 / 8 lanes, orbits at 1.6 volume diagonals:
- *                        2 255 rays    29 575       114 208        394 885
- *   uint8 64^3, 1 px     41  18  14    174  69  85   518 392 434   1029 1082
- *   uint8 64^3, 2 px     41  18  14     76  43  57   188 208 243    939 1069
- *   uint8 32^3           49  20  17    164  69  86   217 186 227    393  505
- *   uint16 64^3          44  19  16    173  80 109   921 527 543   2188 1468
- *   uint16 128^3, 2 px  108  41  34    119  61  73   245 202 233    733  716
- *   float 48^3          397 113  53    501 153 108   543 279 320    980  734
- *   int16 64^3          358 102  51    404 150 143   555 405 429   1290  965
- *   uint8 nearest       184  61  37    393 117 104   344 235 270    638  589
- *   uint8 clamped       258  57  35    379 120 110   839 338 320   1135  735
+ * exchange costs instructions, which a frame that fills the GPU pays for
+ * unless a pixel spans about a voxel or more: then the lanes of a ray share
+ * cache lines that neighbouring rays do not. Ray-cast us with 1 / 4 / 8 lanes
+ * (orbits at 1.6 volume diagonals; rays in thousands, pixels per voxel as
+ * px_per_voxel estimates them):
+ *                       2.3 rays     30           114 (px)         395 (px)
+ *   uint8 64^3          41  18  14   174  69  85  518 392 (0.5)   1029 1082 (0.9)
+ *   uint8 64^3, LOD 2    41  18  14    76  43  57  188 208 (2.0)    939 1069 (1.8)
+ *   uint8 32^3          49  20  17   164  69  86  217 186 (1.0)    393  505 (1.8)
+ *   uint16 64^3         44  19  16   173  80 109  921 527 (0.5)   2188 1468 (0.9)
+ *   uint16 64^3, LOD 3                              101 112 (2.0)    586  562 (1.8)
+ *   uint16 128^3, LOD 2 108  41  34   119  61  73  245 202 (2.0)    733  716 (1.8)
+ *   float 380^3        397 113  53   501 153 108  543 279 (0.7)    980  734 (1.2)
+ *   float 128^3                       89  42       102 103 (2.0)    236  284 (3.7)
+ *   int16 300^3        358 102  51   404 150 143  555 405 (0.8)   1290  965 (1.6)
+ *   nearest 512^3      184  61  37   393 117 104  344 235 (0.5)    638  589 (0.9)
+ *   nearest 128^3                    133  57       144 157 (2.0)    355  445 (3.7)
+ *   clamped 256^3      258  57  35   379 120 110  839 338 (1.0)   1135  735 (1.8)
+ * and whole frames with 1 / 4 lanes: uint8 32^3, 71 rays, 3.1 px 256 229; int16,
+ * 130 rays, 1.9 px 268 229; uint16 64^3, 380 rays, 2.5 px 590 718.
  * The trilinear uint8 kernels have the fewest loads per sample, so they fill
- * the issue slots with the fewest rays; types with eight loads or with
- * clamped taps gain from the shared cache lines to 400 000 rays and (float,
- * int16, uint16 64^3) beyond, where uint16 128^3 and the nearest filter
- * lose. */
+ * the issue slots with the fewest rays. */
 uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
 {
     if (L.kind != LV_LAUNCH_TILE_GRID || L.tile_w != 8 || L.tile_h != 8 || !L.lookahead)
         return 1;
-    const bool light = V.dtype == LV_DT_UINT8 && V.filter == LV_FILTER_TRILINEAR && !V.edge;
+    /* views cast together fill each other's gaps: they split only as few as
+     * the light kernels do (two small views 217 -> 180 us; three with 200 000
+     * rays in all would go from 338 to 357) */
+    const bool together = rays > candidate_rays(V);
+    const bool light =
+        together || (V.dtype == LV_DT_UINT8 && V.filter == LV_FILTER_TRILINEAR && !V.edge);
     const uint64_t eight = light ? 8192 : V.dtype == LV_DT_UINT16 ? 16384 : 32768;
-    const uint64_t four = light ? 81920 : 409600;
+    /* beyond the rays that fill the GPU anyhow, up to a limit that falls as a
+     * voxel covers more pixels */
+    const float p = V.px_per_voxel;
+    const bool fine = light                              ? !together && p < 1.2f && rays <= 196608
+                      : V.filter == LV_FILTER_TRILINEAR ? p * float(rays) < 800000.0f
+                                                         : p < 1.9f;
+    const uint64_t four = fine ? 409600 : light ? 81920 : 49152;
     return rays <= eight ? 8 : rays <= four ? 4 : 1;
 }
 } // namespace

@@ -919,6 +919,14 @@ lv_status make_ray_view(lv_ctx* ctx, const lv_volume* vol, const lv_tf* tf,
     V.tf_mul = V.dmul * float(tf->n);
     V.tf_add = V.dadd * float(tf->n) - 0.5f;
     V.tf_last = float(tf->n - 1u);
+    /* the finest voxel at the volume's centre (or a little off it for an eye
+     * inside), then coarser levels as the LOD threshold allows */
+    const float dist = std::sqrt(eye[0] * eye[0] + eye[1] * eye[1] + eye[2] * eye[2]);
+    V.px_per_voxel = 0.5f * float(desc.height) * std::fabs(desc.camera.projection[5]) /
+                     (float(V.max_voxel_dim) * std::max(dist, 0.4f));
+    for (uint32_t l = lod.min_lod; l + 1u < info.depth; ++l)
+        if (2.0f * V.px_per_voxel <= lod.screen_space_error)
+            V.px_per_voxel *= 2.0f;
     V.accumulate = 0;
     V.max_base = V.edge ? 0u
                         : (V.N[2] - 2u) * V.N[1] * V.N[0] + (V.N[1] - 2u) * V.N[0] + V.N[0] - 2u;
