@@ -1046,45 +1046,61 @@ uint32_t fixed_pitch(const RayView& V)
  * behind chains of dependent loads, so their samples go to more lanes; the
  * exchange costs instructions, which a frame that fills the GPU pays for
  * unless a pixel spans about a voxel or more: then the lanes of a ray share
- * cache lines that neighbouring rays do not. Ray-cast us with 1 / 4 / 8 lanes
- * (orbits at 1.6 volume diagonals; rays in thousands, pixels per voxel as
+ * cache lines that neighbouring rays do not. Ray-cast us with 1 / 4 / 8 lanes,
+ * orbits at 1.6 volume diagonals, by rays and (pixels per voxel, as
  * px_per_voxel estimates them):
- *                       2.3 rays     30           114 (px)         395 (px)
- *   uint8 64^3          41  18  14   174  69  85  518 392 (0.5)   1029 1082 (0.9)
- *   uint8 64^3, LOD 2    41  18  14    76  43  57  188 208 (2.0)    939 1069 (1.8)
- *   uint8 32^3          49  20  17   164  69  86  217 186 (1.0)    393  505 (1.8)
- *   uint16 64^3         44  19  16   173  80 109  921 527 (0.5)   2188 1468 (0.9)
- *   uint16 64^3, LOD 3                              101 112 (2.0)    586  562 (1.8)
- *   uint16 128^3, LOD 2 108  41  34   119  61  73  245 202 (2.0)    733  716 (1.8)
- *   float 380^3        397 113  53   501 153 108  543 279 (0.7)    980  734 (1.2)
- *   float 128^3                       89  42       102 103 (2.0)    236  284 (3.7)
- *   int16 300^3        358 102  51   404 150 143  555 405 (0.8)   1290  965 (1.6)
- *   nearest 512^3      184  61  37   393 117 104  344 235 (0.5)    638  589 (0.9)
- *   nearest 128^3                    133  57       144 157 (2.0)    355  445 (3.7)
- *   clamped 256^3      258  57  35   379 120 110  839 338 (1.0)   1135  735 (1.8)
- * and whole frames with 1 / 4 lanes: uint8 32^3, 71 rays, 3.1 px 256 229; int16,
- * 130 rays, 1.9 px 268 229; uint16 64^3, 380 rays, 2.5 px 590 718.
- * The trilinear uint8 kernels have the fewest loads per sample, so they fill
- * the issue slots with the fewest rays. */
+ *                    13 600          114 000              395 000
+ *   uint8 64^3       81  32  25 ( .6) 515  365 395 (1.0)  1012 1020 1225 ( .9)
+ *    LOD 2 px        36  18  18 (1.3) 182  184 213 (2.0)   920 1000 1212 (1.8)
+ *   uint8 32^3       87  38  29 ( .6) 213  171 197 (1.0)   389  447  577 (1.8)
+ *   uint16 64^3      87  36  29 ( .6) 883  532 507 (1.0)  2204 1424 1597 ( .9)
+ *    LOD 3 px        39  20  18 (1.3) 100  112 137 (2.0)   591  563  732 (1.8)
+ *   uint16 128^3    122  62  43 ( .6) 247  188 195 (2.0)   718  666  774 (1.8)
+ *   float 380^3     571 155  92 ( .2) 548  265 282 ( .7)   992  669  836 (1.2)
+ *   float 128^3      91  34  28 ( .6) 101  105 132 (2.0)   234  286  394 (3.7)
+ *   int16 300^3     467 135  84 ( .3) 563  387 391 ( .8)  1263  914 1113 (1.6)
+ *   nearest 512^3   399 111  66 ( .2) 340  212 235 ( .5)   615  537  699 ( .9)
+ *   nearest 128^3   146  50  38 ( .6) 146  158 191 (2.0)   354  448  590 (3.7)
+ *   clamped 256^3   265  74  57 ( .3) 867  318 286 (1.0)  1119  689  781 (1.8)
+ * and at 794 000 rays, 1 / 4 lanes: uint16 64^3 2983 2353 (1.3), uint16 128^3
+ * 1010 1097 (1.3), float 380^3 1285 1251 (1.8), int16 1682 1531 (2.2), nearest
+ * 512^3 891 992 (1.3), clamped 1486 1257 (2.6). The trilinear uint8 kernels
+ * have the fewest loads per sample, so they fill the issue slots with the
+ * fewest rays; clamped taps have the longest chains. */
 uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
 {
     if (L.kind != LV_LAUNCH_TILE_GRID || L.tile_w != 8 || L.tile_h != 8 || !L.lookahead)
         return 1;
-    /* views cast together fill each other's gaps: they split only as few as
-     * the light kernels do (two small views 217 -> 180 us; three with 200 000
-     * rays in all would go from 338 to 357) */
-    const bool together = rays > candidate_rays(V);
-    const bool light =
-        together || (V.dtype == LV_DT_UINT8 && V.filter == LV_FILTER_TRILINEAR && !V.edge);
-    const uint64_t eight = light ? 8192 : V.dtype == LV_DT_UINT16 ? 16384 : 32768;
-    /* beyond the rays that fill the GPU anyhow, up to a limit that falls as a
-     * voxel covers more pixels */
-    const float p = V.px_per_voxel;
-    const bool fine = light                              ? !together && p < 1.2f && rays <= 196608
-                      : V.filter == LV_FILTER_TRILINEAR ? p * float(rays) < 800000.0f
-                                                         : p < 1.9f;
-    const uint64_t four = fine ? 409600 : light ? 81920 : 49152;
-    return rays <= eight ? 8 : rays <= four ? 4 : 1;
+    const float p = std::max(V.px_per_voxel, 0.01f), r = float(rays);
+    float eight, four; /* rays up to which that many lanes share a ray */
+    if (rays > candidate_rays(V))
+    {
+        /* views cast together fill each other's gaps: few in all (two small
+         * views 217 -> 180 us; three with 200 000 rays 338 -> 357) */
+        eight = 8192.f;
+        four = 81920.f;
+    }
+    else if (V.filter != LV_FILTER_TRILINEAR)
+    {
+        eight = 32768.f;
+        four = p < 1.2f ? 500000.f : 90000.f;
+    }
+    else if (V.edge)
+    {
+        eight = 100000.f;
+        four = 2000000.f / p;
+    }
+    else if (V.dtype == LV_DT_UINT8)
+    {
+        eight = 16384.f;
+        four = p < 1.25f ? 230000.f : 90000.f;
+    }
+    else
+    {
+        eight = V.dtype == LV_DT_UINT16 ? 16384.f : 32768.f;
+        four = p < 1.4f ? 600000.f : (p < 1.9f ? 800000.f : 500000.f) / p;
+    }
+    return r <= eight ? 8 : r <= four ? 4 : 1;
 }
 } // namespace
 
