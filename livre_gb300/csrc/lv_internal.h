@@ -155,6 +155,7 @@ enum FrameCounter
     FC_KEPT = 9,          /* rendering-set entries left after dropping the
                              ones with an ancestor in the set */
     FC_QUEUE = 10,        /* tile queue head of the single-view ray cast */
+    FC_TICKET = 11,       /* blocks of the residency pass that have finished */
     FC_WORDS = 16
 };
 

@@ -319,8 +319,11 @@ struct Renderer
      * recorded before the selection, `join` after the side work */
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    cudaEvent_t leaf_ready = nullptr;    /* the side stream cleared the leaf grid */
     const uint32_t* pre_order = nullptr; /* this frame's tile order (or null) */
-    bool leaf_cleared = false;           /* the side stream cleared the leaf grid */
+    /* cleared ahead for the frame's first residency pass (the leaf grid on
+     * the side stream); not yet joined: the rest of the side stream's work */
+    bool leaf_cleared = false, counters_cleared = false, side_pending = false;
     /* the selection runs on its own high-priority stream once the previous
      * frame's residency pass has read the visible list (`visible_free`), so
      * a frame queued while the previous one still ray casts selects beside

@@ -147,34 +147,171 @@ __device__ void prune_body(const ResolveView& R, uint32_t first, uint32_t stride
     }
 }
 
+/* The leaf cells of node id, dealt over the lanes of a warp. */
+template <class F>
+__device__ __forceinline__ void for_leaf_cells(const ResolveView& R, uint64_t id, F&& f)
+{
+    const uint32_t sh = R.Lf - nid_level(id), mask = (1u << sh) - 1u;
+    const uint32_t x0 = nid_x(id) << sh, y0 = nid_y(id) << sh, z0 = nid_z(id) << sh;
+    const uint64_t cells = uint64_t(1) << (3u * sh);
+    for (uint64_t c = threadIdx.x & 31u; c < cells; c += 32)
+    {
+        const uint32_t cx = x0 + (uint32_t(c) & mask), cy = y0 + (uint32_t(c >> sh) & mask),
+                       cz = z0 + uint32_t(c >> (2u * sh));
+        if (cx < R.dims[0] && cy < R.dims[1] && cz < R.dims[2])
+            f((uint64_t(cz) * R.dims[1] + cy) * R.dims[0] + cx);
+    }
+}
+
 /* Splats the rendering set into the leaf grid; one warp per entry. */
 __device__ void leaf_fill_body(const ResolveView& R, uint32_t warp, uint32_t nwarps)
 {
     const uint32_t n = min(R.counters[FC_RENDERED], R.render_capacity);
-    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t e = warp; e < n; e += nwarps)
     {
         const uint64_t id = R.render_ids[e];
         if (id == kInvalidNode)
             continue;
-        const uint32_t slot = R.render_slots[e];
-        const uint32_t L = nid_level(id);
-        const uint32_t sh = R.Lf - L;
-        const uint32_t side = 1u << sh;
-        const uint32_t x0 = nid_x(id) << sh, y0 = nid_y(id) << sh,
-                       z0 = nid_z(id) << sh;
-        const uint32_t key = (L << kLeafSlotBits) | (slot & kLeafSlotMask);
-        const uint64_t cells = uint64_t(side) * side * side;
-        for (uint64_t c = lane; c < cells; c += 32)
-        {
-            const uint32_t cx = x0 + uint32_t(c % side);
-            const uint32_t cy = y0 + uint32_t((c / side) % side);
-            const uint32_t cz = z0 + uint32_t(c / (uint64_t(side) * side));
-            if (cx < R.dims[0] && cy < R.dims[1] && cz < R.dims[2])
-                atomicMin(&R.leaf[(uint64_t(cz) * R.dims[1] + cy) * R.dims[0] + cx],
-                          key);
-        }
+        const uint32_t key =
+            (nid_level(id) << kLeafSlotBits) | (R.render_slots[e] & kLeafSlotMask);
+        for_leaf_cells(R, id, [&](uint64_t cell) { atomicMin(&R.leaf[cell], key); });
     }
+}
+
+/* The residency pass of one view with the leaf grid in one launch, a warp
+ * per visible node (resolve_body's rules).
+ *
+ * SYNC: no ancestor fallback. The rendering set is part of the visible cut,
+ * whose nodes do not overlap, so a node's cells are simply stored; the last
+ * block to finish writes the counters, the selection's words and the missing
+ * ids into mapped page-locked host memory, where the host waits for them.
+ * Else a missing node's nearest resident ancestor is splatted, the coarser
+ * level winning, which is what dropping the shadowed entries first would
+ * give; prune_kernel then counts the entries kept. Only the selection's words
+ * go to the host.
+ *
+ * The pass used to be three launches (resolve, read-back, leaf fill), behind
+ * one for the selection's words and a clear of the counters: frames of a
+ * 100^3 volume 63.1 -> 54.9 us, of a 256^3 one at 512 x 512 141 -> 134. */
+template <bool SYNC>
+__global__ void __launch_bounds__(256)
+    residency_kernel(const __grid_constant__ ResolveView R, const uint32_t* __restrict__ sel_words,
+                     uint32_t* h_words, uint64_t* h_missing)
+{
+    __shared__ uint32_t available, missing, max_level, error, last;
+    if (threadIdx.x == 0)
+        available = missing = max_level = error = 0u;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t n = *R.n_visible_ptr;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps)
+    {
+        uint64_t id = R.visible[i];
+        uint32_t L = nid_level(id);
+        const bool inside = L < R.depth && nid_x(id) < (R.root_blocks[0] << L) &&
+                            nid_y(id) < (R.root_blocks[1] << L) &&
+                            nid_z(id) < (R.root_blocks[2] << L);
+        const uint64_t idx =
+            inside ? node_index(R.level_offset, R.root_blocks, id) : R.n_nodes;
+        if (idx >= R.n_nodes)
+        {
+            error = 2u; /* id outside this octree */
+            continue;
+        }
+        int32_t slot = R.node_table[idx];
+        if (slot >= 0)
+        {
+            if (lane == 0)
+            {
+                R.node_stamp[idx] = R.frame;
+                R.view_stamp[idx] = R.view_frame;
+                atomicAdd(&available, 1u);
+                if (SYNC)
+                    atomicMax(&max_level, L + 1u);
+                emit_render(R, id, uint32_t(slot));
+            }
+        }
+        else
+        {
+            if (lane == 0)
+            {
+                atomicAdd(&missing, 1u);
+                const uint32_t m = atomicAdd(&R.counters[FC_MISSING], 1u);
+                if (m < R.missing_capacity)
+                    R.missing[m] = id;
+            }
+            if (SYNC)
+                continue;
+            /* the nearest resident ancestor, emitted once per view (the same
+             * walk in every lane) */
+            while (slot < 0 && L > 0)
+            {
+                --L;
+                id = nid_make(L, nid_x(id) >> 1, nid_y(id) >> 1, nid_z(id) >> 1, nid_t(id));
+                slot = R.node_table[node_index(R.level_offset, R.root_blocks, id)];
+            }
+            if (slot < 0)
+                continue;
+            uint32_t seen = 0;
+            if (lane == 0)
+            {
+                const uint64_t p = node_index(R.level_offset, R.root_blocks, id);
+                /* the exchange comes first: the view stamps and the in-use
+                 * stamps may be the same array */
+                seen = atomicExch(&R.view_stamp[p], R.view_frame) == R.view_frame;
+                if (!seen)
+                    emit_render(R, id, uint32_t(slot));
+                R.node_stamp[p] = R.frame;
+            }
+            if (__shfl_sync(0xFFFFFFFFu, seen, 0))
+                continue; /* splatted by the warp that emitted it */
+        }
+        const uint32_t key = (L << kLeafSlotBits) | (uint32_t(slot) & kLeafSlotMask);
+        if (SYNC)
+            for_leaf_cells(R, id, [&](uint64_t cell) { R.leaf[cell] = key; });
+        else
+            for_leaf_cells(R, id, [&](uint64_t cell) { atomicMin(&R.leaf[cell], key); });
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        if (available)
+        {
+            atomicAdd(&R.counters[FC_AVAILABLE], available);
+            if (SYNC)
+            {
+                atomicAdd(&R.counters[FC_KEPT], available);
+                atomicMax(&R.counters[FC_MAX_LEVEL], max_level);
+            }
+        }
+        if (missing)
+            atomicAdd(&R.counters[FC_NOT_AVAILABLE], missing);
+        if (error)
+            atomicExch(&R.counters[FC_ERROR], error);
+        if (SYNC)
+        {
+            __threadfence();
+            last = atomicAdd(&R.counters[FC_TICKET], 1u) == gridDim.x - 1u;
+        }
+        else
+            last = blockIdx.x == 0;
+    }
+    __syncthreads();
+    if (!last)
+        return;
+    if (threadIdx.x < LV_SELECT_RESULT_WORDS)
+        h_words[FC_WORDS + threadIdx.x] = sel_words[threadIdx.x];
+    if (SYNC)
+    {
+        __threadfence();
+        if (threadIdx.x < FC_WORDS)
+            h_words[threadIdx.x] = __ldcg(R.counters + threadIdx.x);
+        const uint32_t n_ids = min(__ldcg(R.counters + FC_MISSING), R.missing_capacity);
+        for (uint32_t i = threadIdx.x; i < n_ids; i += blockDim.x)
+            h_missing[i] = __ldcg(R.missing + i);
+    }
+    __threadfence_system();
 }
 
 __global__ void resolve_kernel(ResolveView R)
@@ -184,11 +321,6 @@ __global__ void resolve_kernel(ResolveView R)
 __global__ void prune_kernel(ResolveView R)
 {
     prune_body(R, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-}
-__global__ void leaf_fill_kernel(ResolveView R)
-{
-    leaf_fill_body(R, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                   (gridDim.x * blockDim.x) >> 5);
 }
 /* multi-view variants: blockIdx.y selects the view */
 __global__ void resolve_views_kernel(const ResolveView* __restrict__ Rs)
@@ -854,14 +986,19 @@ lv_status launch_resolve(lv_ctx* ctx, const ResolveView& R, cudaStream_t s)
     return LV_OK;
 }
 
-lv_status launch_leaf_fill(lv_ctx* ctx, const ResolveView& R, cudaStream_t s)
+lv_status launch_residency(lv_ctx* ctx, const ResolveView& R, const uint32_t* sel_words,
+                           uint32_t* h_words, uint64_t* h_missing, cudaStream_t s)
 {
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    if (!R.synchronous) /* ancestors may shadow entries: drop them */
-        prune_kernel<<<sms, 256, 0, s>>>(R);
-    LV_CUDA(ctx, cudaGetLastError());
-    leaf_fill_kernel<<<2 * sms, 256, 0, s>>>(R);
+    if (R.synchronous)
+        residency_kernel<true><<<sms, 256, 0, s>>>(R, sel_words, h_words, h_missing);
+    else
+    {
+        residency_kernel<false><<<sms, 256, 0, s>>>(R, sel_words, h_words, h_missing);
+        LV_CUDA(ctx, cudaGetLastError());
+        prune_kernel<<<sms, 256, 0, s>>>(R); /* ancestors may shadow entries */
+    }
     LV_CUDA(ctx, cudaGetLastError());
     return LV_OK;
 }

@@ -44,7 +44,8 @@ lv_status launch_blob_bricks(lv_ctx* ctx, const lv_volume_info& v,
                              const uint64_t* d_ids, uint32_t n, uint8_t* out,
                              const uint64_t* d_offsets, cudaStream_t stream);
 lv_status launch_resolve(lv_ctx* ctx, const ResolveView& R, cudaStream_t s);
-lv_status launch_leaf_fill(lv_ctx* ctx, const ResolveView& R, cudaStream_t s);
+lv_status launch_residency(lv_ctx* ctx, const ResolveView& R, const uint32_t* sel_words,
+                           uint32_t* h_words, uint64_t* h_missing, cudaStream_t s);
 lv_status launch_raycast(lv_ctx* ctx, const RayView& V, cudaStream_t s);
 
 namespace
@@ -66,22 +67,6 @@ __global__ void words_to_host_kernel(const uint32_t* __restrict__ src, uint32_t*
 {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
         dst[i] = src[i];
-    __threadfence_system();
-}
-
-/* A synchronous frame's counters and its missing list (as many ids as the
- * residency pass appended, at most cap) into mapped page-locked host
- * memory: the host learns which bricks to stream when it learns how many,
- * without a copy queued behind the frame's first ray cast. */
-__global__ void counters_to_host_kernel(const uint32_t* __restrict__ counters,
-                                        const uint64_t* __restrict__ missing, uint32_t* words,
-                                        uint64_t* ids, uint32_t cap)
-{
-    const uint32_t n = min(counters[FC_MISSING], cap);
-    if (blockIdx.x == 0 && threadIdx.x < FC_WORDS)
-        words[threadIdx.x] = counters[threadIdx.x];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        ids[i] = missing[i];
     __threadfence_system();
 }
 
@@ -336,6 +321,7 @@ lv_status ensure_renderer(lv_ctx* ctx)
     cudaEventCreateWithFlags(&r->resolve_done, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&r->join, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&r->leaf_ready, cudaEventDisableTiming);
     cudaStreamCreateWithFlags(&r->side, cudaStreamNonBlocking);
     {
         int least = 0, greatest = 0;
@@ -1024,6 +1010,7 @@ extern "C" void lv_ctx_destroy(lv_ctx* ctx)
         cudaEventDestroy(ctx->renderer->resolve_done);
         cudaEventDestroy(ctx->renderer->fork);
         cudaEventDestroy(ctx->renderer->join);
+        cudaEventDestroy(ctx->renderer->leaf_ready);
         cudaStreamDestroy(ctx->renderer->side);
         cudaStreamDestroy(ctx->renderer->sel_stream);
         cudaEventDestroy(ctx->renderer->sel_done);
@@ -1509,7 +1496,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     /* the side stream's work for this frame may start from here */
     LV_CUDA(ctx, cudaEventRecord(R.fork, s));
     R.pre_order = nullptr;
-    R.leaf_cleared = false;
+    R.leaf_cleared = R.counters_cleared = R.side_pending = false;
     struct ClearOrder
     {
         Renderer& r;
@@ -1572,17 +1559,16 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     LV.out_ids = R.visible.as<uint64_t>();
     LV.capacity = uint32_t(std::min<uint64_t>(R.visible_capacity, 0xFFFFFFFFu));
     LV.result = R.sel_result.as<uint32_t>();
-    /* kernels: the selection (one cooperative launch, or roots + one per
-     * level + finish) and the copy of its result words to the host; then
-     * resolve, the copy of its counters (synchronous mode) or prune
-     * (asynchronous mode), leaf fill, ray cast (+ tile keys and order when
-     * longest first) and the final copy of the counters. A synchronous frame
-     * that streams misses resolves once more, and leaf fills and ray casts
-     * again if its first ray cast was already queued. */
+    /* kernels: the selection (one launch, or roots + one per level +
+     * finish), the residency pass with the leaf grid (and, in asynchronous
+     * mode, the count of the entries kept), the ray cast (+ tile
+     * keys and order when longest first) and the final copy of the counters.
+     * A synchronous frame that streams misses runs the residency pass once
+     * more, and ray casts again if its first ray cast was already queued. */
     const lv_render_launch& RL = ctx->launch;
     const uint32_t order_launches =
         RL.kind != LV_LAUNCH_GRID && RL.order == LV_ORDER_LONGEST_FIRST ? 2u : 0u;
-    const uint32_t tail_launches = 3u + 1u + order_launches + 1u;
+    const uint32_t tail_launches = (desc->synchronous ? 1u : 2u) + order_launches + 2u;
     /* the selection waits only for the previous frame's residency pass; while
      * that frame may still ray cast, the one-launch cooperative form (whose
      * CTAs must all be resident at once) gives way to the per-level form */
@@ -1602,7 +1588,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     st = scratch_acquire(ctx, ctx->sel, ss); /* after any lv_select_visible */
     if (st != LV_OK)
         return st;
-    R.launches = selection_launches(ctx, 1, info.depth, !overlap) + 1u + tail_launches;
+    R.launches = selection_launches(ctx, 1, info.depth, !overlap) + tail_launches;
     LV_CUDA(ctx, cudaEventRecord(R.t_sel0, ss));
     st = run_selection(ctx, &LV, 1, info.depth, ss, !overlap);
     if (st != LV_OK)
@@ -1615,15 +1601,13 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         if (st != LV_OK)
             return st;
     }
-    /* the frame's selection words for lv_last_stats, copied now: the next
-     * frame's selection may overwrite them before this frame ends */
     st = scratch_release(ctx, ctx->sel, ss);
     if (st != LV_OK)
         return st;
-    st = words_to_host(ctx, R.sel_result.ptr, R.h_counters, FC_WORDS, LV_SELECT_RESULT_WORDS, ss);
-    if (st != LV_OK)
-        return st;
     LV_CUDA(ctx, cudaEventRecord(R.sel_done, ss));
+    /* cleared while the selection runs */
+    LV_CUDA(ctx, cudaMemsetAsync(R.counters.ptr, 0, sizeof(uint32_t) * FC_WORDS, s));
+    R.counters_cleared = true;
     LV_CUDA(ctx, cudaStreamWaitEvent(s, R.sel_done, 0));
 
     /* 2. residency */
@@ -1660,9 +1644,11 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         return st;
     /* from the camera alone, beside the selection: the cleared leaf grid, the
      * pixels no ray of which can reach the volume and the longest-first tile
-     * order of the others; the leaf fill waits for them */
+     * order of the others; the residency pass waits for the first, the ray
+     * cast for all */
     LV_CUDA(ctx, cudaStreamWaitEvent(R.side, R.fork, 0));
     LV_CUDA(ctx, cudaMemsetAsync(R.leaf.ptr, 0xFF, cells * sizeof(uint32_t), R.side));
+    LV_CUDA(ctx, cudaEventRecord(R.leaf_ready, R.side));
     st = shrink_to_candidates(ctx, V, R.side);
     if (st != LV_OK)
         return st;
@@ -1670,7 +1656,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     if (st != LV_OK)
         return st;
     LV_CUDA(ctx, cudaEventRecord(R.join, R.side));
-    R.leaf_cleared = true;
+    R.leaf_cleared = R.side_pending = true;
     /* residency pass, leaf grid and ray cast. The synchronous mode reads the
      * residency pass's miss count back while the rest runs, streams any
      * misses and renders again, and returns without waiting for the ray
@@ -1684,9 +1670,23 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
                                  .count();
         return r;
     };
+    /* the first residency pass of the frame finds the counters and the leaf
+     * grid cleared ahead; a later one (a frame rendered again, a later pass)
+     * clears them itself */
     auto resolve = [&]() -> lv_status {
-        LV_CUDA(ctx, cudaMemsetAsync(R.counters.ptr, 0, sizeof(uint32_t) * FC_WORDS, s));
-        const lv_status t = launch_resolve(ctx, RV, s);
+        if (!R.counters_cleared)
+            LV_CUDA(ctx, cudaMemsetAsync(R.counters.ptr, 0, sizeof(uint32_t) * FC_WORDS, s));
+        R.counters_cleared = false;
+        if (R.leaf_cleared)
+            LV_CUDA(ctx, cudaStreamWaitEvent(s, R.leaf_ready, 0));
+        else
+            LV_CUDA(ctx, cudaMemsetAsync(R.leaf.ptr, 0xFF, cells * sizeof(uint32_t), s));
+        R.leaf_cleared = false;
+        /* the selection's words go to the host with it: the next frame's
+         * selection may overwrite them before this frame ends */
+        const lv_status t =
+            launch_residency(ctx, RV, R.sel_result.as<uint32_t>(), R.h_counters.as_dev<uint32_t>(),
+                             R.h_missing.as_dev<uint64_t>(), s);
         if (t != LV_OK)
             return t;
         /* the next frame's selection may overwrite the visible list now */
@@ -1695,20 +1695,11 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         return LV_OK;
     };
     auto after_resolve = [&]() -> lv_status {
-        /* the first leaf fill of the frame waits for the side stream; a later
-         * one (a frame rendered again, a later pass) clears the grid itself */
-        if (R.leaf_cleared)
-        {
+        if (R.side_pending)
             LV_CUDA(ctx, cudaStreamWaitEvent(s, R.join, 0));
-            R.leaf_cleared = false;
-        }
-        else
-            LV_CUDA(ctx, cudaMemsetAsync(R.leaf.ptr, 0xFF, cells * sizeof(uint32_t), s));
-        lv_status t = launch_leaf_fill(ctx, RV, s);
-        if (t != LV_OK)
-            return t;
+        R.side_pending = false;
         LV_CUDA(ctx, cudaEventRecord(R.t_ray0, s));
-        t = launch_raycast(ctx, V, s);
+        const lv_status t = launch_raycast(ctx, V, s);
         if (t != LV_OK)
             return t;
         LV_CUDA(ctx, cudaEventRecord(R.t_ray1, s));
@@ -1821,9 +1812,9 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         agg.n_passes = passes;
         R.pass_stats = agg;
         R.passes = passes;
-        /* per pass: a residency pass, then resolve, leaf fill and ray cast */
-        R.launches = selection_launches(ctx, 1, info.depth, !overlap) + 1u + order_launches +
-                     passes * 4u;
+        /* per pass: resolve for its misses, then residency pass and ray cast */
+        R.launches = selection_launches(ctx, 1, info.depth, !overlap) + order_launches +
+                     passes * 3u;
         return LV_OK;
     };
     /* A frame queued while the previous one still ray casts (a fly-through
@@ -1891,11 +1882,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         st = resolve();
         if (st != LV_OK)
             return st;
-        /* the counters and the missing ids, through the host mapping */
-        counters_to_host_kernel<<<8, 256, 0, s>>>(
-            R.counters.as<uint32_t>(), R.missing.as<uint64_t>(), R.h_counters.as_dev<uint32_t>(),
-            R.h_missing.as_dev<uint64_t>(), RV.missing_capacity);
-        LV_CUDA(ctx, cudaGetLastError());
+        /* the counters, selection words and missing ids are on the host then */
         LV_CUDA(ctx, cudaEventRecord(R.resolve_done, s));
         /* a volume that streamed last frame likely misses again: then the
          * ray cast waits for the streaming instead of running twice (unless
@@ -1919,9 +1906,8 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
             st = multipass(n_vis, per_pass, ++R.frame);
             if (st != LV_OK)
                 return st;
-            /* this residency pass and its counters' copy, and the leaf fill
-             * and ray cast queued behind them */
-            R.launches += queued ? 4u : 2u;
+            /* this residency pass, and the ray cast queued behind it */
+            R.launches += queued ? 2u : 1u;
         }
         else
         {
@@ -1940,10 +1926,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
                 /* resolve again with the streamed bricks; what still misses
                  * (pool too small) is not rendered */
                 st = frame_tail();
-                if (queued)
-                    R.launches += 3u;
-                else
-                    R.launches += 1; /* one more residency pass */
+                R.launches += queued ? 2u : 1u; /* one more residency pass */
             }
             vol->streamed_last = R.stats.n_uploaded > 0;
         }
