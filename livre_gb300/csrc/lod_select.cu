@@ -371,6 +371,9 @@ __device__ __forceinline__ uint32_t solo_levels(const LodView& V, uint32_t max_d
                                                 uint32_t* __restrict__ counts,
                                                 uint32_t capacity)
 {
+    /* a block alone (the octree has no wider level) leaves the global words
+     * alone, which its launch did not clear */
+    const bool alone = gridDim.x == 1;
     __shared__ uint64_t nodes[2][kSoloItems];
     __shared__ uint32_t count[2], visited, found, max_level, overflowed;
     const uint32_t ry = V.root_blocks[1], rz = V.root_blocks[2];
@@ -455,11 +458,18 @@ __device__ __forceinline__ uint32_t solo_levels(const LodView& V, uint32_t max_d
     }
     if (threadIdx.x == 0)
     {
-        if (l < max_depth)
-            counts[l] = n;
-        uint32_t* overflow = counts + kMaxLevels + 1;
-        if (overflowed)
-            *overflow = 1u;
+        if (alone)
+        {
+            V.result[LV_SEL_WRITTEN] = min(found, V.capacity);
+            V.result[LV_SEL_OVERFLOW] = overflowed;
+        }
+        else
+        {
+            if (l < max_depth)
+                counts[l] = n;
+            if (overflowed)
+                counts[kMaxLevels + 1] = 1u;
+        }
         V.result[LV_SEL_VISITED] = visited;
         V.result[LV_SEL_FOUND] = found;
         V.result[LV_SEL_MAX_LEVEL] = max_level;
@@ -490,7 +500,7 @@ __global__ void __launch_bounds__(256)
     const bool solo = n_roots <= kSoloItems;
     if (blockIdx.x == 0)
     {
-        if (threadIdx.x == 0)
+        if (threadIdx.x == 0 && gridDim.x > 1)
             counts[0] = n_roots;
         if (threadIdx.x < LV_SELECT_RESULT_WORDS)
             V.result[threadIdx.x] = 0u;
@@ -510,6 +520,8 @@ __global__ void __launch_bounds__(256)
         {
             __syncthreads(); /* the zeroed result before solo_levels writes it */
             l = solo_levels(V, max_depth, n_roots, ids0, view0, ids1, view1, counts, capacity);
+            if (gridDim.x == 1)
+                return;
             if (threadIdx.x == 0)
                 *solo_end = l;
         }
@@ -772,6 +784,7 @@ lv_status scratch_release(lv_ctx* ctx, SelectScratch& S, cudaStream_t s)
         LV_CUDA(ctx, cudaEventCreateWithFlags(&S.free_event, cudaEventDisableTiming));
     LV_CUDA(ctx, cudaEventRecord(S.free_event, s));
     S.free_recorded = true;
+    S.free_stream = nullptr;
     return LV_OK;
 }
 
@@ -797,7 +810,6 @@ lv_status run_selection(lv_ctx* ctx, const LodView* host_views,
         if (V.root_blocks[0] * V.root_blocks[1] * V.root_blocks[2] > cap)
             return fail(ctx, LV_ENOMEM, "root frontier exceeds scratch capacity");
         uint32_t* counts = S.counts.as<uint32_t>();
-        LV_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(uint32_t) * (kMaxLevels + 8), stream));
         uint64_t* ids0 = S.ids[0].as<uint64_t>();
         uint64_t* ids1 = S.ids[1].as<uint64_t>();
         uint32_t* view0 = S.view[0].as<uint32_t>();
@@ -810,7 +822,8 @@ lv_status run_selection(lv_ctx* ctx, const LodView* host_views,
         /* (one CTA visits every level of an octree that small by itself) */
         const uint32_t used =
             widest <= kSoloItems ? 1u
-                                 : uint32_t(std::min<uint64_t>(grid, (widest + 255) / 256));
+                                 : std::max(2u, uint32_t(std::min<uint64_t>(
+                                                    grid, (widest + 255) / 256)));
         uint32_t spin = kSpinLimit, absent = 0xFFFFFFFFu;
         if (ctx->test_barrier_polls && used > 1)
         {
@@ -820,12 +833,14 @@ lv_status run_selection(lv_ctx* ctx, const LodView* host_views,
         }
         if (used == 1)
         {
-            /* nothing to be resident with: an ordinary launch */
+            /* nothing to be resident with, no counts to share: an ordinary
+             * launch without a clear */
             lod_fused_kernel<<<1, 256, 0, stream>>>(V, max_depth, ids0, view0, ids1, view1, counts,
                                                     cap, spin, absent);
             LV_CUDA(ctx, cudaGetLastError());
             return LV_OK;
         }
+        LV_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(uint32_t) * (kMaxLevels + 8), stream));
         void* args[] = {&V, &max_depth, &ids0, &view0, &ids1, &view1, &counts,
                         const_cast<uint32_t*>(&cap), &spin, &absent};
         LV_CUDA(ctx, cudaLaunchCooperativeKernel(reinterpret_cast<void*>(lod_fused_kernel),

@@ -127,6 +127,9 @@ struct SelectScratch
      * stream it ran: the next user, on any stream, waits for it */
     cudaEvent_t free_event = nullptr;
     bool free_recorded = false;
+    /* the library's own stream that it was last recorded on (null: another):
+     * work on that stream follows without a wait */
+    cudaStream_t free_stream = nullptr;
     SelectScratch() = default;
     SelectScratch(const SelectScratch&) = delete;
     SelectScratch& operator=(const SelectScratch&) = delete;
@@ -214,11 +217,12 @@ struct RayLaunch
     uint32_t lanes;
 };
 /* Restricts V's rect to the pixels whose ray can reach the volume (its screen
- * rectangle) and clears the others on `s`, beside the selection, so that the
- * ray cast launches no blocks for them (85 % of the pixels of a 1080p orbit
- * frame). Frame times: a float volume at 1001 x 701 477 -> 449 us, the nearest
- * filter at 1024 x 768 406 -> 391, 2048^3 uint8 at 1080p 277 -> 274. */
-lv_status shrink_to_candidates(lv_ctx* ctx, RayView& V, cudaStream_t s);
+ * rectangle) and clears on `s`, in one launch, the frame's counters, its leaf
+ * grid of `cells` cells and the pixels left out; records `ready` when the
+ * first two are done. more: the pixels got a launch of their own behind it,
+ * for which the ray cast must wait. */
+lv_status launch_frame_clear(lv_ctx* ctx, RayView& V, uint64_t cells, cudaStream_t s,
+                             cudaEvent_t ready, bool& more);
 /* Pixels of V whose ray can reach the volume (its screen rectangle within
  * the rendered rect). */
 uint64_t candidate_rays(const RayView& V);
@@ -312,24 +316,22 @@ struct Renderer
      * before its ray cast ends, so the next frame (on any stream) and any
      * brick streaming wait for it */
     cudaEvent_t frame_done = nullptr;
-    /* the residency pass's counters have reached the host */
-    cudaEvent_t resolve_done = nullptr;
     /* work a frame needs from the camera alone (the tile order, clearing
      * the leaf grid) runs on `side` while the selection runs: `fork` is
      * recorded before the selection, `join` after the side work */
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-    cudaEvent_t leaf_ready = nullptr;    /* the side stream cleared the leaf grid */
+    cudaEvent_t clear_done = nullptr;    /* the side stream's frame_clear */
     const uint32_t* pre_order = nullptr; /* this frame's tile order (or null) */
-    /* cleared ahead for the frame's first residency pass (the leaf grid on
-     * the side stream); not yet joined: the rest of the side stream's work */
-    bool leaf_cleared = false, counters_cleared = false, side_pending = false;
+    /* cleared ahead for the frame's first residency pass; not yet joined:
+     * work the side stream does for the ray cast */
+    bool cleared = false, side_pending = false;
     /* the selection runs on its own high-priority stream once the previous
      * frame's residency pass has read the visible list (`visible_free`), so
      * a frame queued while the previous one still ray casts selects beside
-     * it; `sel_done` orders the rest of the frame after it */
+     * it; the scratch's free_event orders the rest of the frame after it */
     cudaStream_t sel_stream = nullptr;
-    cudaEvent_t sel_done = nullptr, visible_free = nullptr;
+    cudaEvent_t visible_free = nullptr;
     bool visible_free_recorded = false;
     /* timing of the last frame: selection and ray cast */
     cudaEvent_t t_sel0 = nullptr, t_sel1 = nullptr, t_ray0 = nullptr, t_ray1 = nullptr;

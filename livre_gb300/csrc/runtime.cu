@@ -318,17 +318,15 @@ lv_status ensure_renderer(lv_ctx* ctx)
     cudaEventCreateWithFlags(&r->expand_done, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&r->gather_done, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&r->frame_done, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&r->resolve_done, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&r->join, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&r->leaf_ready, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&r->clear_done, cudaEventDisableTiming);
     cudaStreamCreateWithFlags(&r->side, cudaStreamNonBlocking);
     {
         int least = 0, greatest = 0;
         cudaDeviceGetStreamPriorityRange(&least, &greatest);
         cudaStreamCreateWithPriority(&r->sel_stream, cudaStreamNonBlocking, greatest);
     }
-    cudaEventCreateWithFlags(&r->sel_done, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&r->visible_free, cudaEventDisableTiming);
     cudaEventCreate(&r->t_sel0);
     cudaEventCreate(&r->t_sel1);
@@ -1007,13 +1005,11 @@ extern "C" void lv_ctx_destroy(lv_ctx* ctx)
         cudaEventDestroy(ctx->renderer->expand_done);
         cudaEventDestroy(ctx->renderer->gather_done);
         cudaEventDestroy(ctx->renderer->frame_done);
-        cudaEventDestroy(ctx->renderer->resolve_done);
         cudaEventDestroy(ctx->renderer->fork);
         cudaEventDestroy(ctx->renderer->join);
-        cudaEventDestroy(ctx->renderer->leaf_ready);
+        cudaEventDestroy(ctx->renderer->clear_done);
         cudaStreamDestroy(ctx->renderer->side);
         cudaStreamDestroy(ctx->renderer->sel_stream);
-        cudaEventDestroy(ctx->renderer->sel_done);
         cudaEventDestroy(ctx->renderer->visible_free);
         cudaEventDestroy(ctx->renderer->t_sel0);
         cudaEventDestroy(ctx->renderer->t_sel1);
@@ -1496,7 +1492,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     /* the side stream's work for this frame may start from here */
     LV_CUDA(ctx, cudaEventRecord(R.fork, s));
     R.pre_order = nullptr;
-    R.leaf_cleared = R.counters_cleared = R.side_pending = false;
+    R.cleared = R.side_pending = false;
     struct ClearOrder
     {
         Renderer& r;
@@ -1585,9 +1581,12 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
      * residency pass is done; otherwise in stream order */
     overlap = overlap && R.visible_free_recorded;
     LV_CUDA(ctx, cudaStreamWaitEvent(ss, overlap ? R.visible_free : R.fork, 0));
-    st = scratch_acquire(ctx, ctx->sel, ss); /* after any lv_select_visible */
-    if (st != LV_OK)
-        return st;
+    if (ctx->sel.free_stream != ss) /* after any lv_select_visible */
+    {
+        st = scratch_acquire(ctx, ctx->sel, ss);
+        if (st != LV_OK)
+            return st;
+    }
     R.launches = selection_launches(ctx, 1, info.depth, !overlap) + tail_launches;
     LV_CUDA(ctx, cudaEventRecord(R.t_sel0, ss));
     st = run_selection(ctx, &LV, 1, info.depth, ss, !overlap);
@@ -1604,11 +1603,8 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     st = scratch_release(ctx, ctx->sel, ss);
     if (st != LV_OK)
         return st;
-    LV_CUDA(ctx, cudaEventRecord(R.sel_done, ss));
-    /* cleared while the selection runs */
-    LV_CUDA(ctx, cudaMemsetAsync(R.counters.ptr, 0, sizeof(uint32_t) * FC_WORDS, s));
-    R.counters_cleared = true;
-    LV_CUDA(ctx, cudaStreamWaitEvent(s, R.sel_done, 0));
+    ctx->sel.free_stream = ss;
+    LV_CUDA(ctx, cudaStreamWaitEvent(s, ctx->sel.free_event, 0));
 
     /* 2. residency */
     ResolveView RV;
@@ -1642,21 +1638,21 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
                        R.counters.as<uint32_t>(), V);
     if (st != LV_OK)
         return st;
-    /* from the camera alone, beside the selection: the cleared leaf grid, the
-     * pixels no ray of which can reach the volume and the longest-first tile
-     * order of the others; the residency pass waits for the first, the ray
-     * cast for all */
+    /* from the camera alone, beside the selection: the cleared counters, leaf
+     * grid and pixels no ray of which can reach the volume, then the
+     * longest-first tile order of the others; the residency pass waits for
+     * the first, the ray cast for all */
     LV_CUDA(ctx, cudaStreamWaitEvent(R.side, R.fork, 0));
-    LV_CUDA(ctx, cudaMemsetAsync(R.leaf.ptr, 0xFF, cells * sizeof(uint32_t), R.side));
-    LV_CUDA(ctx, cudaEventRecord(R.leaf_ready, R.side));
-    st = shrink_to_candidates(ctx, V, R.side);
+    st = launch_frame_clear(ctx, V, cells, R.side, R.clear_done, R.side_pending);
     if (st != LV_OK)
         return st;
+    R.cleared = true;
     st = prepare_frame_order(ctx, V, ctx->launch, R.side, R.pre_order);
     if (st != LV_OK)
         return st;
-    LV_CUDA(ctx, cudaEventRecord(R.join, R.side));
-    R.leaf_cleared = R.side_pending = true;
+    R.side_pending = R.side_pending || R.pre_order;
+    if (R.side_pending)
+        LV_CUDA(ctx, cudaEventRecord(R.join, R.side));
     /* residency pass, leaf grid and ray cast. The synchronous mode reads the
      * residency pass's miss count back while the rest runs, streams any
      * misses and renders again, and returns without waiting for the ray
@@ -1674,14 +1670,14 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
      * grid cleared ahead; a later one (a frame rendered again, a later pass)
      * clears them itself */
     auto resolve = [&]() -> lv_status {
-        if (!R.counters_cleared)
-            LV_CUDA(ctx, cudaMemsetAsync(R.counters.ptr, 0, sizeof(uint32_t) * FC_WORDS, s));
-        R.counters_cleared = false;
-        if (R.leaf_cleared)
-            LV_CUDA(ctx, cudaStreamWaitEvent(s, R.leaf_ready, 0));
+        if (R.cleared)
+            LV_CUDA(ctx, cudaStreamWaitEvent(s, R.clear_done, 0));
         else
+        {
+            LV_CUDA(ctx, cudaMemsetAsync(R.counters.ptr, 0, sizeof(uint32_t) * FC_WORDS, s));
             LV_CUDA(ctx, cudaMemsetAsync(R.leaf.ptr, 0xFF, cells * sizeof(uint32_t), s));
-        R.leaf_cleared = false;
+        }
+        R.cleared = false;
         /* the selection's words go to the host with it: the next frame's
          * selection may overwrite them before this frame ends */
         const lv_status t =
@@ -1882,8 +1878,8 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         st = resolve();
         if (st != LV_OK)
             return st;
-        /* the counters, selection words and missing ids are on the host then */
-        LV_CUDA(ctx, cudaEventRecord(R.resolve_done, s));
+        /* the counters, selection words and missing ids are on the host once
+         * visible_free has completed */
         /* a volume that streamed last frame likely misses again: then the
          * ray cast waits for the streaming instead of running twice (unless
          * this frame's misses were streamed beside the previous frame).
@@ -1898,7 +1894,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
             if (st != LV_OK)
                 return st;
         }
-        LV_CUDA(ctx, cudaEventSynchronize(R.resolve_done));
+        LV_CUDA(ctx, cudaEventSynchronize(R.visible_free));
         const uint32_t n_vis = hc[FC_WORDS + LV_SEL_WRITTEN];
         if (per_pass > 0 && n_vis > per_pass)
         {
