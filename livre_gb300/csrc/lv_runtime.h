@@ -360,6 +360,9 @@ struct Renderer
     PinnedBuffer h_gather;
     cudaEvent_t gather_done = nullptr;
     bool gather_recorded = false;
+    /* lv_histogram: its jobs (mapped), counts and the accumulated ones' copy */
+    PinnedBuffer h_hist_jobs, h_hist_acc;
+    DeviceBuffer hist_out;
 };
 
 
