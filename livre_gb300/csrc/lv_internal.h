@@ -98,9 +98,8 @@ struct RayView
     uint32_t n_clip;
     uint32_t dims[3]; /* leaf grid (finest level) */
     uint32_t Lf;      /* finest level = depth - 1 */
-    uint32_t N[3], B[3], O[3];
+    uint32_t N[3];    /* voxels per row, column and stack of a brick */
     uint32_t dtype;   /* lv_dtype */
-    uint32_t bpv;     /* bytes per voxel */
     uint32_t filter;
     uint32_t edge;    /* 1: some overlap is 0, clamp every trilinear tap */
     uint32_t quads;   /* bricks stored as voxel quads (quad_layout) */

@@ -846,13 +846,11 @@ lv_status make_ray_view(lv_ctx* ctx, const lv_volume* vol, const lv_tf* tf,
         V.goff[a] = half * V.gscale[a];
         V.dims[a] = dims[a];
         V.N[a] = info.max_block[a];
-        V.O[a] = info.overlap[a];
-        V.B[a] = info.max_block[a] - 2u * info.overlap[a];
         V.f0[a] = std::fma(V.eye[a], V.gscale[a], V.goff[a]);
         V.cell_hi[a] = dims[a] == bm ? float(dims[a]) - 0.5f : 4194304.0f;
         V.cube_end[a] = dims[a] == bm ? std::numeric_limits<float>::infinity() : float(dims[a]);
-        V.Bf[a] = float(V.B[a]);
-        V.Oh[a] = float(V.O[a]) - (desc.filter == LV_FILTER_TRILINEAR ? 0.5f : 0.0f);
+        V.Bf[a] = float(info.max_block[a] - 2u * info.overlap[a]);
+        V.Oh[a] = float(info.overlap[a]) - (desc.filter == LV_FILTER_TRILINEAR ? 0.5f : 0.0f);
         if (info.overlap[a] == 0 || V.N[a] < 2)
             V.edge = 1;
     }
@@ -861,7 +859,6 @@ lv_status make_ray_view(lv_ctx* ctx, const lv_volume* vol, const lv_tf* tf,
     std::memcpy(V.clip, lod.clip_planes, sizeof(V.clip));
     V.Lf = Lf;
     V.dtype = info.dtype;
-    V.bpv = bytes_per_voxel(info.dtype);
     V.quads = vol->stage_off != 0;
     V.filter = desc.filter == LV_FILTER_TRILINEAR ? LV_FILTER_TRILINEAR : LV_FILTER_NEAREST;
     /* the transfer function's range when valid, else the type's
