@@ -485,7 +485,10 @@ lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
  * (every brick resident, no L2 flush), against 0.239 ms for 8 x 16 tiles,
  * 0.31 ms without look-ahead, 0.28 ms in raster order, 0.35 ms for warp
  * tiles and 0.37 ms for the persistent tile queue; and the friendliest to
- * other work on the device (no resident grid).
+ * other work on the device (no resident grid). Under it, frames of few rays
+ * are cast with 4 or 8 lanes per ray in tiles of 4 x 4 or 4 x 2 pixels: the
+ * same image and sample count, 90 us against 208 us of ray casting (256^3
+ * uint8 in 32^3 bricks at 512 x 512).
  * No reference counterpart (the reference rasterises one brick at a time,
  * RayCastRenderer.cpp:503-571). */
 enum
