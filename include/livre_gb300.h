@@ -155,6 +155,11 @@ lv_status lv_select_visible_host(lv_ctx* ctx, const lv_volume_info* vol,
  * 1 .. 2^22. */
 lv_status lv_test_fail_grid_barrier(lv_ctx* ctx, uint32_t polls);
 
+/* Test hook of lv_render's error returns: the context's next lv_render
+ * returns LV_EDEVICE once it has queued the clear of the frame's pixels that
+ * no ray reaches, as a failed allocation there would make it return. */
+lv_status lv_test_fail_frame(lv_ctx* ctx);
+
 /* LOD selection that allocates nothing, for callers that cannot allocate
  * device memory (a host application whose own caching allocator owns the
  * GPU's memory, or a per-frame path that must not risk the device-wide

@@ -158,6 +158,7 @@ struct lv_ctx
     lv::SelectScratch sel;
     lv::DeviceBuffer sel_host_out; /* lv_select_visible_host's device output */
     uint32_t test_barrier_polls = 0; /* lv_test_fail_grid_barrier */
+    bool test_fail_frame = false;    /* lv_test_fail_frame */
     lv::Pool* pool = nullptr;
     lv::Renderer* renderer = nullptr;
     size_t pool_bytes = size_t(3072) << 20;
@@ -323,8 +324,9 @@ struct Renderer
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaEvent_t clear_done = nullptr;    /* the side stream's frame_clear */
     const uint32_t* pre_order = nullptr; /* this frame's tile order (or null) */
-    /* cleared ahead for the frame's first residency pass; not yet joined:
-     * work the side stream does for the ray cast */
+    /* cleared ahead for the frame's first residency pass (until that pass has
+     * waited for the clear); not yet joined: work the side stream does for the
+     * ray cast */
     bool cleared = false, side_pending = false;
     /* the selection runs on its own high-priority stream once the previous
      * frame's residency pass has read the visible list (`visible_free`), so

@@ -1464,6 +1464,15 @@ extern "C" lv_status lv_get_render_launch(lv_ctx* ctx, lv_render_launch* cfg)
     return LV_OK;
 }
 
+extern "C" lv_status lv_test_fail_frame(lv_ctx* ctx)
+{
+    if (!ctx)
+        return LV_EINVAL;
+    std::lock_guard<std::mutex> lock(ctx->mutex);
+    ctx->test_fail_frame = true;
+    return LV_OK;
+}
+
 extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
                                const lv_render_desc* desc, float* d_rgba,
                                void* stream)
@@ -1490,11 +1499,22 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     LV_CUDA(ctx, cudaEventRecord(R.fork, s));
     R.pre_order = nullptr;
     R.cleared = R.side_pending = false;
-    struct ClearOrder
+    /* On every way out the caller's stream has waited for the side stream: its
+     * clear writes the caller's frame, which a caller may reuse in stream
+     * order after an error too. A frame that was queued has waited already. */
+    struct SideWork
     {
         Renderer& r;
-        ~ClearOrder() { r.pre_order = nullptr; }
-    } clear_order{R};
+        cudaStream_t s;
+        ~SideWork()
+        {
+            if ((r.cleared || r.side_pending) &&
+                cudaEventRecord(r.join, r.side) == cudaSuccess)
+                cudaStreamWaitEvent(s, r.join, 0);
+            r.cleared = r.side_pending = false;
+            r.pre_order = nullptr;
+        }
+    } side_work{R, s};
     /* async: bricks missed by the previous frame are streamed now */
     if (!desc->synchronous)
     {
@@ -1640,13 +1660,18 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
      * longest-first tile order of the others; the residency pass waits for
      * the first, the ray cast for all */
     LV_CUDA(ctx, cudaStreamWaitEvent(R.side, R.fork, 0));
+    R.cleared = true; /* from here on `s` waits for the side stream */
     st = launch_frame_clear(ctx, V, cells, R.side, R.clear_done, R.side_pending);
     if (st != LV_OK)
         return st;
-    R.cleared = true;
     st = prepare_frame_order(ctx, V, ctx->launch, R.side, R.pre_order);
     if (st != LV_OK)
         return st;
+    if (ctx->test_fail_frame)
+    {
+        ctx->test_fail_frame = false;
+        return fail(ctx, LV_EDEVICE, "frame failed on request (lv_test_fail_frame)");
+    }
     R.side_pending = R.side_pending || R.pre_order;
     if (R.side_pending)
         LV_CUDA(ctx, cudaEventRecord(R.join, R.side));
