@@ -263,6 +263,9 @@ enum
 lv_status lv_volume_create_blob(lv_ctx* ctx, const lv_volume_info* info,
                                 const lv_blob_desc* blob, uint32_t placement,
                                 lv_volume** out);
+/* Destroys a volume and gives back its bricks. No frame, batch or request on it
+ * may be unfinished: lv_render and lv_batch_render have returned (their device
+ * work is waited for here), and lv_server_wait has returned for every request. */
 void lv_volume_destroy(lv_volume* vol);
 /* The derived VolumeInformation of a volume. */
 lv_status lv_volume_get_info(const lv_volume* vol, lv_volume_info* out);

@@ -574,10 +574,13 @@ class Context:
         return int(out.value)
 
     def close(self):
-        """Destroys the volumes and transfer functions of this context, then it
-        (the C ABI requires children to go first)."""
+        """Destroys the servers and batches of this context, which render its
+        volumes, then the volumes and transfer functions, then it (the C ABI
+        requires children to go first)."""
         if self.handle:
-            for child in list(self._children):
+            for child in sorted(self._children,
+                                key=lambda c: 0 if isinstance(c, Server) else
+                                1 if isinstance(c, Batch) else 2):
                 child.close()
             lib().lv_ctx_destroy(self.handle)
             self.handle = None

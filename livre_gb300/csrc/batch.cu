@@ -107,6 +107,7 @@ struct lv_batch
     uint32_t frame = 0;
     /* previous launch, for the async misses and for statistics */
     std::vector<lv_batch_view> last;
+    std::vector<std::weak_ptr<char>> last_alive; /* of the views' volumes */
     bool pending = false;
     uint64_t uploaded_bytes = 0;
     uint32_t uploaded = 0;
@@ -292,8 +293,8 @@ lv_status process_misses(lv_batch* b)
         const uint32_t m = std::min<uint32_t>(
             std::min<uint32_t>(c[FC_MISSING], uint32_t(b->missing_stride)),
             b->last[i].desc.max_uploads);
-        if (!m)
-            continue;
+        if (!m || b->last_alive[i].expired())
+            continue; /* nothing missed, or the volume is gone */
         uint32_t loaded = 0;
         uint64_t bytes = 0;
         lv_status st = stream_bricks(ctx, b->last[i].volume, miss + b->missing_stride * i, m,
@@ -1017,6 +1018,9 @@ extern "C" lv_status lv_batch_render(lv_batch* b, const lv_batch_view* views, ui
     LV_CUDA(ctx, cudaStreamWaitEvent(user, b->done, 0));
     b->last_n = n_run;
     b->last.assign(views, views + n);
+    b->last_alive.clear();
+    for (uint32_t i = 0; i < n; ++i)
+        b->last_alive.push_back(views[i].volume->alive);
     b->pending = true;
     /* selection: roots + levels + finish; resolve, prune, leaf, step; per
      * non-empty group one persistent launch (+ key and order passes) */

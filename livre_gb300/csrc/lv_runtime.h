@@ -12,6 +12,7 @@
 #include <cstring>
 #include <list>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -476,6 +477,10 @@ struct lv_volume
     /* host pin counts per node: bricks of admitted, unfinished server
      * requests are never evicted (empty until a server uses the volume) */
     std::vector<uint16_t> pins;
+    /* expires, under the context's mutex, when the volume is destroyed: what
+     * outlives a request or a batch (a server's pins, a batch's misses) holds
+     * a weak reference and leaves a destroyed volume alone */
+    std::shared_ptr<char> alive = std::make_shared<char>();
     uint32_t time_step = 0;
     /* the last synchronous frame streamed bricks: the next one likely will
      * too, so it waits for its miss count before queueing the ray cast */

@@ -1264,6 +1264,7 @@ extern "C" void lv_volume_destroy(lv_volume* v)
         cudaSetDevice(ctx->device);
         cudaDeviceSynchronize();
         drop_volume_residency(ctx, v);
+        v->alive.reset();
         if (ctx->renderer && ctx->renderer->pending_vol == v)
             ctx->renderer->pending_vol = nullptr;
         if (ctx->renderer && ctx->renderer->last_vol == v)

@@ -67,6 +67,15 @@ void CUDART_CB stamp_done(void* p)
     static_cast<DoneClock*>(p)->t.store(now_ms());
 }
 
+/* The bricks an admitted request pins. The request may be collected, and its
+ * volume destroyed, between its view's hook and the batch's completion. */
+struct Pins
+{
+    lv_volume* volume;
+    std::weak_ptr<char> alive;
+    std::vector<uint64_t> nodes;
+};
+
 struct Inflight
 {
     lv_batch* batch = nullptr;
@@ -74,7 +83,7 @@ struct Inflight
      * hook may be collected (and freed) by lv_server_wait before the batch
      * ends */
     std::vector<uint64_t> tickets;
-    std::vector<std::pair<lv_volume*, std::vector<uint64_t>>> pins;
+    std::vector<Pins> pins;
     lv_status status = LV_OK;
     cudaEvent_t ev = nullptr;
     std::shared_ptr<DoneClock> clock;
@@ -139,10 +148,12 @@ void complete(lv_server* S, Inflight& f)
         lv_batch_stats(f.batch, st.data(), n, &batch_ms, &ray_ms);
     {
         std::lock_guard<std::mutex> lk(S->ctx->mutex);
-        for (auto& vp : f.pins)
+        for (const Pins& p : f.pins)
         {
-            lv_volume* v = vp.first;
-            for (uint64_t idx : vp.second)
+            if (p.alive.expired())
+                continue; /* its pins went with the volume */
+            lv_volume* v = p.volume;
+            for (uint64_t idx : p.nodes)
                 if (v->pins[idx] && --v->pins[idx] == 0 && v->host_table[idx] >= 0)
                     --S->ctx->pool->pinned_count[v->slot_units];
         }
@@ -530,7 +541,7 @@ void loop_batched(lv_server* S)
         for (Req* r : admitted)
         {
             f.tickets.push_back(r->ticket);
-            f.pins.emplace_back(r->r.volume, std::move(r->pinned));
+            f.pins.push_back({r->r.volume, r->r.volume->alive, std::move(r->pinned)});
             r->pinned.clear();
         }
         {
