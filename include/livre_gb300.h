@@ -446,7 +446,8 @@ typedef struct lv_frame_stats
     uint32_t n_uploaded;      /* bricks streamed into the pool */
     uint64_t n_samples;       /* composited samples */
     uint64_t bytes_uploaded;  /* host->device brick bytes */
-    uint32_t n_launches;      /* kernels this library launched for the frame */
+    uint32_t n_launches;      /* kernels this library launched for the frame,
+                                 those that streamed its bricks included */
     float select_ms;          /* device time of the LOD selection */
     float raycast_ms;         /* device time of the ray-cast kernel */
     uint32_t error_flags;     /* 0, or the device's index-check code: 1 rendering

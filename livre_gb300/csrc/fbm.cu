@@ -475,9 +475,9 @@ lv_status launch_fbm_bricks(lv_ctx* ctx, const lv_volume_info& info, const lv_fb
                             uint8_t* out, const uint64_t* d_offsets, uint64_t brick_bytes,
                             cudaStream_t s)
 {
-    for (uint32_t first = 0; first < n; first += 65535u)
+    for (uint32_t first = 0; first < n; first += kFbmLaunchBricks)
     {
-        const uint32_t cnt = std::min(65535u, n - first);
+        const uint32_t cnt = std::min(kFbmLaunchBricks, n - first);
         constexpr int R = 8;
         const uint32_t runs =
             (info.max_block[0] + R - 1) / R * info.max_block[1] * info.max_block[2];

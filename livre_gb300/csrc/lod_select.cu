@@ -788,11 +788,6 @@ lv_status scratch_release(lv_ctx* ctx, SelectScratch& S, cudaStream_t s)
     return LV_OK;
 }
 
-uint32_t selection_launches(lv_ctx* ctx, uint32_t n_views, uint32_t depth, bool allow_fused)
-{
-    return allow_fused && n_views == 1 && fused_grid(ctx) ? 1u : depth + 2u;
-}
-
 lv_status run_selection(lv_ctx* ctx, const LodView* host_views,
                         uint32_t n_views, uint32_t max_depth,
                         cudaStream_t stream, bool allow_fused)
@@ -837,6 +832,7 @@ lv_status run_selection(lv_ctx* ctx, const LodView* host_views,
              * launch without a clear */
             lod_fused_kernel<<<1, 256, 0, stream>>>(V, max_depth, ids0, view0, ids1, view1, counts,
                                                     cap, spin, absent);
+            ++ctx->kernels;
             LV_CUDA(ctx, cudaGetLastError());
             return LV_OK;
         }
@@ -845,6 +841,7 @@ lv_status run_selection(lv_ctx* ctx, const LodView* host_views,
                         const_cast<uint32_t*>(&cap), &spin, &absent};
         LV_CUDA(ctx, cudaLaunchCooperativeKernel(reinterpret_cast<void*>(lod_fused_kernel),
                                                  dim3(used), dim3(256), args, 0, stream));
+        ++ctx->kernels;
         return LV_OK;
     }
     LV_CUDA(ctx, S.staging.reserve(sizeof(LodView) * n_views));
@@ -895,6 +892,7 @@ lv_status enqueue_selection(lv_ctx* ctx, SelectScratch& S, const LodView* dviews
     }
     lod_finish_kernel<<<(n_views + 127) / 128, 128, 0, stream>>>(dviews, n_views,
                                                                  overflow);
+    ctx->kernels += max_depth + 2u;
     LV_CUDA(ctx, cudaGetLastError());
     return LV_OK;
 }
@@ -945,9 +943,13 @@ lv_status range_slice(lv_ctx* ctx, const lv_volume_info& vol,
                                           vol.root_blocks[2], keys, vals, n_pad);
     for (uint32_t k = 2; k <= n_pad; k <<= 1)
         for (uint32_t j = k >> 1; j > 0; j >>= 1)
+        {
             bitonic_pass_kernel<<<nb, tb, 0, stream>>>(keys, vals, n_pad, j, k);
+            ++ctx->kernels;
+        }
     slice_kernel<<<1, 256, 0, stream>>>(vals, d_ids, d_result, range[0],
                                         range[1]);
+    ctx->kernels += 2u; /* with the keys' */
     LV_CUDA(ctx, cudaGetLastError());
     return LV_OK;
 }

@@ -169,6 +169,9 @@ struct lv_ctx
     /* host fetchers of callback sources (created on first use) */
     lv::HostPool* host_pool = nullptr;
     lv_ctx_totals totals{}; /* since creation, host-side (lv_get_totals) */
+    /* kernels launched under the mutex, counted where they are launched: a
+     * frame's n_launches is what it added */
+    uint64_t kernels = 0;
     /* bumped by every pool user other than lv_render (batches, the server)
      * whose work may still read pool slots when it returns */
     std::atomic<uint64_t> foreign_pool_use{0};
@@ -228,6 +231,8 @@ lv_status launch_frame_clear(lv_ctx* ctx, RayView& V, uint64_t cells, cudaStream
 /* Pixels of V whose ray can reach the volume (its screen rectangle within
  * the rendered rect). */
 uint64_t candidate_rays(const RayView& V);
+/* Bricks a launch of the fBm generator makes at most. */
+constexpr uint32_t kFbmLaunchBricks = 65535;
 /* The launch the ray cast of V uses under L when `rays` candidate rays are
  * cast at once (V's own, or those of all views of a batch). */
 RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays);
@@ -235,10 +240,6 @@ RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays)
  * renderer's tile scratch (null for raster order or the per-pixel grid). */
 lv_status prepare_frame_order(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
                               cudaStream_t side, const uint32_t*& order);
-
-/* Kernels run_selection launches for n views of an octree of `depth` levels. */
-uint32_t selection_launches(lv_ctx* ctx, uint32_t n_views, uint32_t depth,
-                            bool allow_fused = true);
 
 /* Enqueues the selection kernels for n views whose constants are already
  * on the device (capturable: no host synchronisation). */

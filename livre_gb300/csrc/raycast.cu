@@ -1008,6 +1008,7 @@ lv_status launch_resolve(lv_ctx* ctx, const ResolveView& R, cudaStream_t s)
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     resolve_kernel<<<sms, 256, 0, s>>>(R);
+    ++ctx->kernels;
     LV_CUDA(ctx, cudaGetLastError());
     return LV_OK;
 }
@@ -1024,7 +1025,9 @@ lv_status launch_residency(lv_ctx* ctx, const ResolveView& R, const uint32_t* se
         residency_kernel<false><<<sms, 256, 0, s>>>(R, sel_words, h_words, h_missing);
         LV_CUDA(ctx, cudaGetLastError());
         prune_kernel<<<sms, 256, 0, s>>>(R); /* ancestors may shadow entries */
+        ++ctx->kernels;
     }
+    ++ctx->kernels;
     LV_CUDA(ctx, cudaGetLastError());
     return LV_OK;
 }
@@ -1134,6 +1137,7 @@ const uint32_t* tile_order(lv_ctx* ctx, const RayView& V, const lv_render_launch
     tile_key_kernel<<<blocks, 256, 0, s>>>(V, L.tile_w, L.tile_h, tiles_x, total, per_length,
                                            keys, hist);
     tile_order_kernel<<<blocks, 256, 0, s>>>(keys, hist, order, total);
+    ctx->kernels += 2u;
     e = cudaGetLastError();
     if (e != cudaSuccess)
     {
@@ -1213,6 +1217,7 @@ lv_status launch_frame_clear(lv_ctx* ctx, RayView& V, uint64_t cells, cudaStream
     LV_CUDA(ctx, cudaEventRecord(ready, s));
     if (more)
         clear_outside_kernel<<<clear_grid(C), 256, 0, s>>>(C);
+    ctx->kernels += more ? 2u : 1u;
     LV_CUDA(ctx, cudaGetLastError());
     return LV_OK;
 }
@@ -1555,6 +1560,7 @@ lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const RayLaunch& R,
                               uint8_t* order_scratch, cudaStream_t s)
 {
     const lv_render_launch& L = R.shape;
+    ++ctx->kernels; /* whichever launch it is */
     const bool other = V.dtype != LV_DT_UINT8 && V.dtype != LV_DT_UINT16;
     if (other || R.lanes > 1)
     {

@@ -201,6 +201,7 @@ lv_status words_to_host(lv_ctx* ctx, const void* d_src, const PinnedBuffer& host
 {
     words_to_host_kernel<<<1, 32, 0, s>>>(static_cast<const uint32_t*>(d_src),
                                           static_cast<uint32_t*>(host.dev) + word_offset, n);
+    ++ctx->kernels;
     LV_CUDA(ctx, cudaGetLastError());
     return LV_OK;
 }
@@ -461,6 +462,7 @@ lv_status apply_updates(
         const uint32_t n = uint32_t(kv.second.size() / 2);
         scatter_kernel<<<(n + 255) / 256, 256, 0, s>>>(
             kv.first->node_table.as<int32_t>(), R.pairs.as<int64_t>() + off, n);
+        ++ctx->kernels;
         off += kv.second.size();
     }
     LV_CUDA(ctx, cudaGetLastError());
@@ -647,6 +649,7 @@ lv_status stream_bricks(lv_ctx* ctx, lv_volume* vol, const uint64_t* ids,
                                      dids.as<uint64_t>() + gen_ids.size(), up);
         if (g != LV_OK)
             return g;
+        ctx->kernels += vol->kind == SRC_FBM_DEVICE ? (gen_ids.size() + kFbmLaunchBricks - 1) / kFbmLaunchBricks : 1u;
     }
     if (!gather.empty())
     {
@@ -667,6 +670,7 @@ lv_status stream_bricks(lv_ctx* ctx, lv_volume* vol, const uint64_t* ids,
             arena, vol->host_store.as_dev<uint8_t>(), static_cast<const uint64_t*>(R.h_gather.dev),
             uint32_t(vol->brick_bytes), vol->info.max_block[0], vol->info.max_block[1],
             vol->stage_off != 0);
+        ++ctx->kernels;
         LV_CUDA(ctx, cudaGetLastError());
         LV_CUDA(ctx, cudaEventRecord(R.gather_done, up));
         R.gather_recorded = true;
@@ -682,6 +686,7 @@ lv_status stream_bricks(lv_ctx* ctx, lv_volume* vol, const uint64_t* ids,
         expand_quads_kernel<<<uint32_t(expand.size()), kExpandThreads, 0, up>>>(
             arena, static_cast<const uint64_t*>(R.h_expand.dev), vol->info.max_block[0],
             vol->info.max_block[1], voxels, uint32_t(vol->stage_off));
+        ++ctx->kernels;
         LV_CUDA(ctx, cudaGetLastError());
         LV_CUDA(ctx, cudaEventRecord(R.expand_done, up));
         R.expand_recorded = true;
@@ -1490,6 +1495,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     Renderer& R = *ctx->renderer;
     const lv_volume_info& info = vol->info;
 
+    const uint64_t kernels_before = ctx->kernels;
     lv_frame_stats stats{};
     R.stats = stats;
     /* the previous frame's buffers are reused: its work (maybe on another
@@ -1533,6 +1539,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         drop_volume_residency(ctx, vol);
         std::fill(vol->host_table.begin(), vol->host_table.end(), -1);
         fill_i32_kernel<<<256, 256, 0, s>>>(vol->node_table.as<int32_t>(), vol->n_nodes, -1);
+        ++ctx->kernels;
         vol->time_step = desc->lod.time_step;
     }
 
@@ -1573,16 +1580,6 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     LV.out_ids = R.visible.as<uint64_t>();
     LV.capacity = uint32_t(std::min<uint64_t>(R.visible_capacity, 0xFFFFFFFFu));
     LV.result = R.sel_result.as<uint32_t>();
-    /* kernels: the selection (one launch, or roots + one per level +
-     * finish), the residency pass with the leaf grid (and, in asynchronous
-     * mode, the count of the entries kept), the ray cast (+ tile
-     * keys and order when longest first) and the final copy of the counters.
-     * A synchronous frame that streams misses runs the residency pass once
-     * more, and ray casts again if its first ray cast was already queued. */
-    const lv_render_launch& RL = ctx->launch;
-    const uint32_t order_launches =
-        RL.kind != LV_LAUNCH_GRID && RL.order == LV_ORDER_LONGEST_FIRST ? 2u : 0u;
-    const uint32_t tail_launches = (desc->synchronous ? 1u : 2u) + order_launches + 2u;
     /* the selection waits only for the previous frame's residency pass; while
      * that frame may still ray cast, the one-launch cooperative form (whose
      * CTAs must all be resident at once) gives way to the per-level form */
@@ -1605,7 +1602,6 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         if (st != LV_OK)
             return st;
     }
-    R.launches = selection_launches(ctx, 1, info.depth, !overlap) + tail_launches;
     LV_CUDA(ctx, cudaEventRecord(R.t_sel0, ss));
     st = run_selection(ctx, &LV, 1, info.depth, ss, !overlap);
     if (st != LV_OK)
@@ -1831,9 +1827,6 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         agg.n_passes = passes;
         R.pass_stats = agg;
         R.passes = passes;
-        /* per pass: resolve for its misses, then residency pass and ray cast */
-        R.launches = selection_launches(ctx, 1, info.depth, !overlap) + order_launches +
-                     passes * 3u;
         return LV_OK;
     };
     /* A frame queued while the previous one still ray casts (a fly-through
@@ -1856,8 +1849,8 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
         LV_CUDA(ctx, cudaMemsetAsync(R.probe_count.ptr, 0, sizeof(uint32_t), ss));
         probe_kernel<<<256, 256, 0, ss>>>(RV, R.probe.as<uint64_t>(), R.probe_count.as<uint32_t>(),
                                           cap);
+        ++ctx->kernels;
         LV_CUDA(ctx, cudaGetLastError());
-        ++R.launches;
         uint32_t* hcount = R.h_probe.as<uint32_t>();
         uint64_t* hids = R.h_probe.as<uint64_t>() + 1;
         LV_CUDA(ctx, cudaMemcpyAsync(hcount, R.probe_count.ptr, sizeof(uint32_t),
@@ -1925,8 +1918,6 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
             st = multipass(n_vis, per_pass, ++R.frame);
             if (st != LV_OK)
                 return st;
-            /* this residency pass, and the ray cast queued behind it */
-            R.launches += queued ? 2u : 1u;
         }
         else
         {
@@ -1945,7 +1936,6 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
                 /* resolve again with the streamed bricks; what still misses
                  * (pool too small) is not rendered */
                 st = frame_tail();
-                R.launches += queued ? 2u : 1u; /* one more residency pass */
             }
             vol->streamed_last = R.stats.n_uploaded > 0;
         }
@@ -1979,6 +1969,7 @@ extern "C" lv_status lv_render(lv_ctx* ctx, lv_volume* vol, lv_tf* tf,
     R.last_vol = vol;
     R.last_desc = *desc;
     R.foreign_seen = ctx->foreign_pool_use.load();
+    R.launches = uint32_t(ctx->kernels - kernels_before);
     ++ctx->totals.frames;
     ctx->totals.bricks_uploaded += R.stats.n_uploaded;
     ctx->totals.bytes_uploaded += R.stats.bytes_uploaded;
