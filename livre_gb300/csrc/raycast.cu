@@ -981,8 +981,13 @@ __global__ void __launch_bounds__(256)
     const uint64_t t = (uint64_t(blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < FC_WORDS)
         counters[t] = 0u;
-    for (uint64_t i = t; i < cells; i += uint64_t(gridDim.x) * gridDim.y * blockDim.x)
-        leaf[i] = kLeafEmpty;
+    /* four cells a store: the grid is a device allocation */
+    const uint64_t threads = uint64_t(gridDim.x) * gridDim.y * blockDim.x;
+    for (uint64_t i = t; i < cells / 4u; i += threads)
+        reinterpret_cast<uint4*>(leaf)[i] =
+            make_uint4(kLeafEmpty, kLeafEmpty, kLeafEmpty, kLeafEmpty);
+    if (t < (cells & 3u))
+        leaf[(cells & ~uint64_t(3)) + t] = kLeafEmpty;
     if (C.W)
         clear_pixels(C);
 }
@@ -1210,8 +1215,15 @@ lv_status launch_frame_clear(lv_ctx* ctx, RayView& V, uint64_t cells, cudaStream
     ClearRect now = C;
     if (more)
         now.W = 0;
-    const dim3 grid = now.W ? clear_grid(now)
-                            : dim3(uint32_t(std::min<uint64_t>((cells + 1023) / 1024, 608u)));
+    /* enough blocks for the larger of the two jobs: a narrow rect of a deep
+     * octree has few pixels and many cells */
+    const uint32_t for_cells = uint32_t(std::min<uint64_t>((cells + 1023) / 1024, 608u));
+    dim3 grid(for_cells);
+    if (now.W)
+    {
+        grid = clear_grid(now);
+        grid.y = std::max(grid.y, (for_cells + grid.x - 1) / grid.x);
+    }
     frame_clear_kernel<<<grid, 256, 0, s>>>(V.counters, const_cast<uint32_t*>(V.leaf), cells, now);
     LV_CUDA(ctx, cudaGetLastError());
     LV_CUDA(ctx, cudaEventRecord(ready, s));
