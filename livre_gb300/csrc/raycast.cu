@@ -116,28 +116,30 @@ __device__ void resolve_body(const ResolveView& R, uint32_t first, uint32_t stri
     }
 }
 
-/* Drops rendering-set entries that have an ancestor in the set, as
- * RenderingSetGenerator::generateRenderingSet does (RenderingSetGeneratorFilter
- * .cpp:63-79): every entry of this view carries view_stamp == view_frame. */
+/* A rendering-set entry that has an ancestor in the set: every entry of this
+ * view carries view_stamp == view_frame. */
+__device__ __forceinline__ bool shadowed(const ResolveView& R, uint64_t id)
+{
+    while (nid_level(id) > 0)
+    {
+        id = nid_make(nid_level(id) - 1u, nid_x(id) >> 1, nid_y(id) >> 1, nid_z(id) >> 1,
+                      nid_t(id));
+        if (R.view_stamp[node_index(R.level_offset, R.root_blocks, id)] == R.view_frame)
+            return true;
+    }
+    return false;
+}
+
+/* Drops shadowed rendering-set entries, as
+ * RenderingSetGenerator::generateRenderingSet does
+ * (RenderingSetGeneratorFilter.cpp:63-79). */
 __device__ void prune_body(const ResolveView& R, uint32_t first, uint32_t stride)
 {
     const uint32_t n = min(R.counters[FC_RENDERED], R.render_capacity);
     for (uint32_t e = first; e < n; e += stride)
     {
         const uint64_t id = R.render_ids[e];
-        uint64_t cur = id;
-        bool shadowed = false;
-        while (nid_level(cur) > 0)
-        {
-            cur = nid_make(nid_level(cur) - 1u, nid_x(cur) >> 1, nid_y(cur) >> 1,
-                           nid_z(cur) >> 1, nid_t(cur));
-            if (R.view_stamp[node_index(R.level_offset, R.root_blocks, cur)] == R.view_frame)
-            {
-                shadowed = true;
-                break;
-            }
-        }
-        if (shadowed)
+        if (shadowed(R, id))
             R.render_ids[e] = kInvalidNode;
         else
         {
@@ -147,52 +149,66 @@ __device__ void prune_body(const ResolveView& R, uint32_t first, uint32_t stride
     }
 }
 
-/* The leaf cells of node id, dealt over the lanes of a warp. */
+/* The cells of the leaf grid under node id that fall to part `part` of
+ * `parts`, dealt over the lanes of a warp. (A grid has at most 2^28 cells.) */
 template <class F>
-__device__ __forceinline__ void for_leaf_cells(const ResolveView& R, uint64_t id, F&& f)
+__device__ __forceinline__ void for_leaf_cells(const ResolveView& R, uint64_t id, uint32_t part,
+                                               uint32_t parts, F&& f)
 {
-    const uint32_t sh = R.Lf - nid_level(id), mask = (1u << sh) - 1u;
+    const uint32_t sh = R.Lf - nid_level(id), mask = (1u << sh) - 1u, cells = 1u << (3u * sh);
     const uint32_t x0 = nid_x(id) << sh, y0 = nid_y(id) << sh, z0 = nid_z(id) << sh;
-    const uint64_t cells = uint64_t(1) << (3u * sh);
-    for (uint64_t c = threadIdx.x & 31u; c < cells; c += 32)
+    for (uint32_t c = 32u * part + (threadIdx.x & 31u); c < cells; c += 32u * parts)
     {
-        const uint32_t cx = x0 + (uint32_t(c) & mask), cy = y0 + (uint32_t(c >> sh) & mask),
-                       cz = z0 + uint32_t(c >> (2u * sh));
-        if (cx < R.dims[0] && cy < R.dims[1] && cz < R.dims[2])
-            f((uint64_t(cz) * R.dims[1] + cy) * R.dims[0] + cx);
+        const uint32_t x = x0 + (c & mask), y = y0 + ((c >> sh) & mask), z = z0 + (c >> (2u * sh));
+        if (x < R.dims[0] && y < R.dims[1] && z < R.dims[2])
+            f((z * R.dims[1] + y) * R.dims[0] + x);
     }
 }
 
-/* Splats the rendering set into the leaf grid; one warp per entry. */
+/* Warps that share a node's cells where n nodes have nwarps warps: the fewer
+ * nodes a frame renders, the more cells each covers. One warp for the 16.7 M
+ * cells under the root of an 8192^3 octree in 32^3 bricks, shown small, made
+ * a frame of 25.9 ms (asynchronous 38.6, with an atomic minimum per cell);
+ * shared it is one of 86 us (93). The root of a 2048^3 octree in 64^3 bricks:
+ * 122 -> 71 us. */
+__device__ __forceinline__ uint32_t cell_parts(uint32_t n, uint32_t nwarps)
+{
+    return n && n < nwarps ? nwarps / n : 1u;
+}
+
+/* Splats the rendering set into the leaf grid, a warp or several per entry. */
 __device__ void leaf_fill_body(const ResolveView& R, uint32_t warp, uint32_t nwarps)
 {
     const uint32_t n = min(R.counters[FC_RENDERED], R.render_capacity);
-    for (uint32_t e = warp; e < n; e += nwarps)
+    const uint32_t parts = cell_parts(n, nwarps);
+    for (uint32_t i = warp; i < n * parts; i += nwarps)
     {
+        const uint32_t e = parts > 1u ? i % n : i;
         const uint64_t id = R.render_ids[e];
         if (id == kInvalidNode)
             continue;
         const uint32_t key =
             (nid_level(id) << kLeafSlotBits) | (R.render_slots[e] & kLeafSlotMask);
-        for_leaf_cells(R, id, [&](uint64_t cell) { atomicMin(&R.leaf[cell], key); });
+        for_leaf_cells(R, id, parts > 1u ? i / n : 0u, parts,
+                       [&](uint32_t cell) { atomicMin(&R.leaf[cell], key); });
     }
 }
 
-/* The residency pass of one view with the leaf grid in one launch, a warp
- * per visible node (resolve_body's rules).
+/* The residency pass of one view, a warp or several per visible node
+ * (resolve_body's rules).
  *
  * SYNC: no ancestor fallback. The rendering set is part of the visible cut,
- * whose nodes do not overlap, so a node's cells are simply stored; the last
- * block to finish writes the counters, the selection's words and the missing
- * ids into mapped page-locked host memory, where the host waits for them.
- * Else a missing node's nearest resident ancestor is splatted, the coarser
- * level winning, which is what dropping the shadowed entries first would
- * give; prune_kernel then counts the entries kept. Only the selection's words
- * go to the host.
+ * whose nodes do not overlap, so the nodes' cells of the leaf grid are simply
+ * stored (cell_parts), and the last block to finish writes the counters, the
+ * selection's words and the missing ids into mapped page-locked host memory,
+ * where the host waits for them. Else a missing node's nearest resident
+ * ancestor is emitted, prune_leaf_kernel drops the entries it shadows and
+ * stores the others' cells, and only the selection's words go to the host.
  *
- * The pass used to be three launches (resolve, read-back, leaf fill), behind
- * one for the selection's words and a clear of the counters: frames of a
- * 100^3 volume 63.1 -> 54.9 us, of a 256^3 one at 512 x 512 141 -> 134. */
+ * The synchronous pass used to be three launches (resolve, read-back, leaf
+ * fill), behind one for the selection's words and a clear of the counters:
+ * frames of a 100^3 volume 63.1 -> 54.9 us, of a 256^3 one at 512 x 512
+ * 141 -> 134. */
 template <bool SYNC>
 __global__ void __launch_bounds__(256)
     residency_kernel(const __grid_constant__ ResolveView R, const uint32_t* __restrict__ sel_words,
@@ -205,9 +221,12 @@ __global__ void __launch_bounds__(256)
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n = *R.n_visible_ptr;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps)
+    const uint32_t parts = SYNC ? cell_parts(n, nwarps) : 1u;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n * parts; i += nwarps)
     {
-        uint64_t id = R.visible[i];
+        const uint32_t part = parts > 1u ? i / n : 0u;
+        const bool lead = lane == 0 && part == 0; /* reports the node */
+        uint64_t id = R.visible[i - part * n];
         uint32_t L = nid_level(id);
         const bool inside = L < R.depth && nid_x(id) < (R.root_blocks[0] << L) &&
                             nid_y(id) < (R.root_blocks[1] << L) &&
@@ -222,7 +241,7 @@ __global__ void __launch_bounds__(256)
         int32_t slot = R.node_table[idx];
         if (slot >= 0)
         {
-            if (lane == 0)
+            if (lead)
             {
                 R.node_stamp[idx] = R.frame;
                 R.view_stamp[idx] = R.view_frame;
@@ -234,7 +253,7 @@ __global__ void __launch_bounds__(256)
         }
         else
         {
-            if (lane == 0)
+            if (lead)
             {
                 atomicAdd(&missing, 1u);
                 const uint32_t m = atomicAdd(&R.counters[FC_MISSING], 1u);
@@ -251,27 +270,21 @@ __global__ void __launch_bounds__(256)
                 id = nid_make(L, nid_x(id) >> 1, nid_y(id) >> 1, nid_z(id) >> 1, nid_t(id));
                 slot = R.node_table[node_index(R.level_offset, R.root_blocks, id)];
             }
-            if (slot < 0)
-                continue;
-            uint32_t seen = 0;
-            if (lane == 0)
+            if (slot >= 0 && lane == 0)
             {
                 const uint64_t p = node_index(R.level_offset, R.root_blocks, id);
                 /* the exchange comes first: the view stamps and the in-use
                  * stamps may be the same array */
-                seen = atomicExch(&R.view_stamp[p], R.view_frame) == R.view_frame;
-                if (!seen)
+                if (atomicExch(&R.view_stamp[p], R.view_frame) != R.view_frame)
                     emit_render(R, id, uint32_t(slot));
                 R.node_stamp[p] = R.frame;
             }
-            if (__shfl_sync(0xFFFFFFFFu, seen, 0))
-                continue; /* splatted by the warp that emitted it */
         }
-        const uint32_t key = (L << kLeafSlotBits) | (uint32_t(slot) & kLeafSlotMask);
         if (SYNC)
-            for_leaf_cells(R, id, [&](uint64_t cell) { R.leaf[cell] = key; });
-        else
-            for_leaf_cells(R, id, [&](uint64_t cell) { atomicMin(&R.leaf[cell], key); });
+        {
+            const uint32_t key = (L << kLeafSlotBits) | (uint32_t(slot) & kLeafSlotMask);
+            for_leaf_cells(R, id, part, parts, [&](uint32_t cell) { R.leaf[cell] = key; });
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -314,13 +327,54 @@ __global__ void __launch_bounds__(256)
     __threadfence_system();
 }
 
+/* The end of an asynchronous residency pass, a warp or several per entry of
+ * the rendering set: drops the entry if it is shadowed, else counts it and
+ * stores its cells of the leaf grid (the entries kept do not overlap). A warp
+ * that finds the entry dropped already leaves it; one that does not comes to
+ * the same answer. */
+__global__ void __launch_bounds__(256)
+    prune_leaf_kernel(const __grid_constant__ ResolveView R)
+{
+    __shared__ uint32_t kept, max_level;
+    if (threadIdx.x == 0)
+        kept = max_level = 0u;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t n = min(R.counters[FC_RENDERED], R.render_capacity);
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, parts = cell_parts(n, nwarps);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n * parts; i += nwarps)
+    {
+        const uint32_t part = parts > 1u ? i / n : 0u, e = i - part * n;
+        const bool lead = lane == 0 && part == 0;
+        const uint64_t id = *static_cast<volatile uint64_t*>(R.render_ids + e);
+        if (__any_sync(0xFFFFFFFFu, id == kInvalidNode))
+            continue;
+        if (shadowed(R, id))
+        {
+            if (lead)
+                R.render_ids[e] = kInvalidNode;
+            continue;
+        }
+        const uint32_t L = nid_level(id);
+        if (lead)
+        {
+            atomicAdd(&kept, 1u);
+            atomicMax(&max_level, L + 1u);
+        }
+        const uint32_t key = (L << kLeafSlotBits) | (R.render_slots[e] & kLeafSlotMask);
+        for_leaf_cells(R, id, part, parts, [&](uint32_t cell) { R.leaf[cell] = key; });
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && kept)
+    {
+        atomicAdd(&R.counters[FC_KEPT], kept);
+        atomicMax(&R.counters[FC_MAX_LEVEL], max_level);
+    }
+}
+
 __global__ void resolve_kernel(ResolveView R)
 {
     resolve_body(R, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-}
-__global__ void prune_kernel(ResolveView R)
-{
-    prune_body(R, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 /* multi-view variants: blockIdx.y selects the view */
 __global__ void resolve_views_kernel(const ResolveView* __restrict__ Rs)
@@ -1029,7 +1083,7 @@ lv_status launch_residency(lv_ctx* ctx, const ResolveView& R, const uint32_t* se
     {
         residency_kernel<false><<<sms, 256, 0, s>>>(R, sel_words, h_words, h_missing);
         LV_CUDA(ctx, cudaGetLastError());
-        prune_kernel<<<sms, 256, 0, s>>>(R); /* ancestors may shadow entries */
+        prune_leaf_kernel<<<sms, 256, 0, s>>>(R);
         ++ctx->kernels;
     }
     ++ctx->kernels;
