@@ -160,6 +160,12 @@ lv_status lv_test_fail_grid_barrier(lv_ctx* ctx, uint32_t polls);
  * no ray reaches, as a failed allocation there would make it return. */
 lv_status lv_test_fail_frame(lv_ctx* ctx);
 
+/* Test hook of the ray cast: `lanes` (1, 4 or 8) lanes share a ray in the
+ * context's lv_render frames under the default launch, whatever their size; 0
+ * gives the choice back to the rule. last (may be null) receives the lanes of
+ * the last frame. */
+lv_status lv_test_ray_lanes(lv_ctx* ctx, uint32_t lanes, uint32_t* last);
+
 /* LOD selection that allocates nothing, for callers that cannot allocate
  * device memory (a host application whose own caching allocator owns the
  * GPU's memory, or a per-frame path that must not risk the device-wide

@@ -164,6 +164,7 @@ _SIGNATURES = {
                                             C.c_uint32, C.c_void_p, C.c_void_p]),
     "lv_test_fail_grid_barrier": (C.c_int, [C.c_void_p, C.c_uint32]),
     "lv_test_fail_frame": (C.c_int, [C.c_void_p]),
+    "lv_test_ray_lanes": (C.c_int, [C.c_void_p, C.c_uint32, P(C.c_uint32)]),
     "lv_select_visible_host": (C.c_int, [C.c_void_p, P(VolumeInfo), P(Camera), P(LodParams),
                                          C.c_void_p, C.c_uint32, C.c_void_p]),
     "lv_pool_configure": (C.c_int, [C.c_void_p, C.c_size_t]),

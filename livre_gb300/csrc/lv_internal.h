@@ -124,7 +124,9 @@ struct RayView
                                a conservative bound of the pixels whose ray can
                                reach the volume's box; the others start and end
                                with no sample */
-    float px_per_voxel;     /* estimated screen size of a rendered voxel's side */
+    /* estimates for the host's choice of launch, at the volume's centre:
+     * screen size of a rendered voxel's side and of a ray's step */
+    float px_per_voxel, px_per_step;
     uint32_t samples_fixed; /* 0 = policy */
     uint32_t step_policy;
     uint32_t max_voxel_dim;

@@ -160,6 +160,7 @@ struct lv_ctx
     lv::DeviceBuffer sel_host_out; /* lv_select_visible_host's device output */
     uint32_t test_barrier_polls = 0; /* lv_test_fail_grid_barrier */
     bool test_fail_frame = false;    /* lv_test_fail_frame */
+    uint32_t test_lanes = 0;         /* lv_test_ray_lanes */
     lv::Pool* pool = nullptr;
     lv::Renderer* renderer = nullptr;
     size_t pool_bytes = size_t(3072) << 20;
@@ -234,8 +235,10 @@ uint64_t candidate_rays(const RayView& V);
 /* Bricks a launch of the fBm generator makes at most. */
 constexpr uint32_t kFbmLaunchBricks = 65535;
 /* The launch the ray cast of V uses under L when `rays` candidate rays are
- * cast at once (V's own, or those of all views of a batch). */
-RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays);
+ * cast at once (V's own, or those of all views of a batch); forced: the lanes
+ * per ray of lv_test_ray_lanes, 0 by the rule. */
+RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays,
+                     uint32_t forced = 0);
 /* lv_render's tile order for V under L, computed on `side` into the
  * renderer's tile scratch (null for raster order or the per-pixel grid). */
 lv_status prepare_frame_order(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
@@ -340,6 +343,7 @@ struct Renderer
     /* timing of the last frame: selection and ray cast */
     cudaEvent_t t_sel0 = nullptr, t_sel1 = nullptr, t_ray0 = nullptr, t_ray1 = nullptr;
     uint32_t launches = 0;
+    uint32_t lanes = 1; /* per ray, of the last frame's ray cast */
     /* multi-pass frames: the visible set split into pool-sized passes */
     PinnedBuffer h_pass;     /* visible ids in pass order */
     DeviceBuffer pass_count; /* visible ids of the current pass */

@@ -1306,38 +1306,53 @@ uint32_t fixed_pitch(const RayView& V)
     return fixed ? V.N[0] : 0;
 }
 
+/* The default launch. */
+bool splittable(const lv_render_launch& L)
+{
+    return L.kind == LV_LAUNCH_TILE_GRID && L.tile_w == 8 && L.tile_h == 8 && L.lookahead;
+}
+
 /* Lanes that share a ray in a launch of `rays` candidate rays (pixels that
  * can reach the volume) under the default launch; other launch shapes keep
  * one lane per ray. Few rays leave most of the 152 SMs' issue slots idle
  * behind chains of dependent loads, so their samples go to more lanes; the
  * exchange costs instructions, which a frame that fills the GPU pays for
- * unless a pixel spans about a voxel or more: then the lanes of a ray share
- * cache lines that neighbouring rays do not. Ray-cast us with 1 / 4 / 8 lanes,
- * orbits at 1.6 volume diagonals, by rays and (pixels per voxel, as
- * px_per_voxel estimates them):
- *                    13 600          114 000              395 000
- *   uint8 64^3       81  32  25 ( .6) 515  365 395 (1.0)  1012 1020 1225 ( .9)
- *    LOD 2 px        36  18  18 (1.3) 182  184 213 (2.0)   920 1000 1212 (1.8)
- *   uint8 32^3       87  38  29 ( .6) 213  171 197 (1.0)   389  447  577 (1.8)
- *   uint16 64^3      87  36  29 ( .6) 883  532 507 (1.0)  2204 1424 1597 ( .9)
- *    LOD 3 px        39  20  18 (1.3) 100  112 137 (2.0)   591  563  732 (1.8)
- *   uint16 128^3    122  62  43 ( .6) 247  188 195 (2.0)   718  666  774 (1.8)
- *   float 380^3     571 155  92 ( .2) 548  265 282 ( .7)   992  669  836 (1.2)
- *   float 128^3      91  34  28 ( .6) 101  105 132 (2.0)   234  286  394 (3.7)
- *   int16 300^3     467 135  84 ( .3) 563  387 391 ( .8)  1263  914 1113 (1.6)
- *   nearest 512^3   399 111  66 ( .2) 340  212 235 ( .5)   615  537  699 ( .9)
- *   nearest 128^3   146  50  38 ( .6) 146  158 191 (2.0)   354  448  590 (3.7)
- *   clamped 256^3   265  74  57 ( .3) 867  318 286 (1.0)  1119  689  781 (1.8)
- * and at 794 000 rays, 1 / 4 lanes: uint16 64^3 2983 2353 (1.3), uint16 128^3
- * 1010 1097 (1.3), float 380^3 1285 1251 (1.8), int16 1682 1531 (2.2), nearest
- * 512^3 891 992 (1.3), clamped 1486 1257 (2.6). The trilinear uint8 kernels
- * have the fewest loads per sample, so they fill the issue slots with the
- * fewest rays; clamped taps have the longest chains. */
+ * unless the samples of a ray share cache lines that neighbouring rays do not:
+ * the ray's step is well below a pixel (px_per_step), a pixel not below a
+ * voxel. Ray-cast us with 1 / 4 / 8 lanes, by rays and (px_per_voxel,
+ * px_per_step), orbits at 1.6 volume diagonals:
+ *                    13 600               114 000                395 000
+ *   uint8 64^3       81  32  25 ( .6, .3) 515  365 395 (1.0, .3)  1012 1020 1225 ( .9,  .5)
+ *    LOD 2 px        36  18  18 (1.3, .6) 182  184 213 (2.0, .5)   920 1000 1212 (1.8,  .5)
+ *   uint8 32^3       87  38  29 ( .6, .3) 213  171 197 (1.0, .5)   389  447  577 (1.8,  .9)
+ *   uint16 64^3      87  36  29 ( .6, .3) 883  532 507 (1.0, .3)  2204 1424 1597 ( .9,  .5)
+ *    LOD 3 px        39  20  18 (1.3, .6) 100  112 137 (2.0, 1.)   591  563  732 (1.8,  .9)
+ *   uint16 128^3    122  62  43 ( .6, .2) 247  188 195 (2.0, .5)   718  666  774 (1.8,  .9)
+ *   float 380^3     571 155  92 ( .2, .1) 548  265 282 ( .7, .3)   992  669  836 (1.2,  .6)
+ *   float 128^3      91  34  28 ( .6, .3) 101  105 132 (2.0, 1.)   234  286  394 (3.7, 1.8)
+ *   int16 300^3     467 135  84 ( .3, .1) 563  387 391 ( .8, .4)  1263  914 1113 (1.6,  .8)
+ *   nearest 512^3   399 111  66 ( .2, .2) 340  212 235 ( .5, .5)   615  537  699 ( .9,  .9)
+ *   nearest 128^3   146  50  38 ( .6, .2) 146  158 191 (2.0, .5)   354  448  590 (3.7,  .9)
+ *   clamped 256^3   265  74  57 ( .3, .2) 867  318 286 (1.0, .5)  1119  689  781 (1.8,  .9)
+ * The trilinear uint8 kernels have the fewest loads per sample, so they fill
+ * the issue slots with the fewest rays; clamped taps have the longest chains.
+ *
+ * uint16 and int8: rays * px_per_step separates what gains from what loses.
+ * Of 1008 uint16 frames (bricks of 16^3 to 128^3, tables of 256 and 4096
+ * entries, orbits and paths inside, both step policies) none with a product
+ * up to 250 000 is over 12 % slower with four lanes than with one, 6 over 3 %
+ * (by limits on rays and px_per_voxel alone 56, the worst 23 %); 1024^3 uint16:
+ * (240 000 rays, .65) 391 / 264, (373 000, .41) 805 / 623, (581 000, .51) 1141
+ * / 1179, inside (173 000, .96) 361 / 283, (307 000, 1.3) 422 / 422, (480 000,
+ * 1.6) 526 / 602; 256^3 int8 (147 000, .5) 223 / 180, (373 000, .8) 334 / 405.
+ * Clamped uint16 2048^3: (373 000, .4) 1133 / 844, (949 000, .33) 4307 / 3742,
+ * (949 000, .65) 2226 / 2558, (2.6 M, .6) 11388 / 14437. */
 uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
 {
-    if (L.kind != LV_LAUNCH_TILE_GRID || L.tile_w != 8 || L.tile_h != 8 || !L.lookahead)
+    if (!splittable(L))
         return 1;
     const float p = std::max(V.px_per_voxel, 0.01f), r = float(rays);
+    const float step = std::max(V.px_per_step, 0.001f);
     float eight, four; /* rays up to which that many lanes share a ray */
     if (rays > candidate_rays(V))
     {
@@ -1354,7 +1369,7 @@ uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
     else if (V.edge)
     {
         eight = 100000.f;
-        four = 2000000.f / p;
+        four = std::min(2000000.f / p, 600000.f / step);
     }
     else if (V.dtype == LV_DT_UINT8)
     {
@@ -1364,15 +1379,17 @@ uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
     else
     {
         eight = V.dtype == LV_DT_UINT16 ? 16384.f : 32768.f;
-        four = p < 1.4f ? 600000.f : (p < 1.9f ? 800000.f : 500000.f) / p;
+        four = V.dtype == LV_DT_UINT16 || V.dtype == LV_DT_INT8
+                   ? 250000.f / step
+                   : p < 1.4f ? 600000.f : (p < 1.9f ? 800000.f : 500000.f) / p;
     }
     return r <= eight ? 8 : r <= four ? 4 : 1;
 }
 } // namespace
 
-RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays)
+RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays, uint32_t forced)
 {
-    RayLaunch R{L, split_lanes(V, L, rays)};
+    RayLaunch R{L, splittable(L) && forced ? forced : split_lanes(V, L, rays)};
     if (R.lanes > 1)
     {
         /* 64 threads: 4 x 4 pixels of 4 lanes or 4 x 2 of 8 */
@@ -1396,7 +1413,7 @@ lv_status prepare_frame_order(lv_ctx* ctx, const RayView& V, const lv_render_lau
                               cudaStream_t side, const uint32_t*& order)
 {
     order = nullptr;
-    const lv_render_launch T = ray_launch(V, L, candidate_rays(V)).shape;
+    const lv_render_launch T = ray_launch(V, L, candidate_rays(V), ctx->test_lanes).shape;
     /* tiles that are all resident at once (64-thread blocks, 12 per SM at
      * least) start together in any order: no order is computed, three launches
      * fewer */
@@ -1619,7 +1636,9 @@ lv_status launch_raycast(lv_ctx* ctx, const RayView& V, cudaStream_t s)
     if (V.dtype > LV_DT_INT32)
         return fail(ctx, LV_EINVAL, "unknown voxel type");
     /* the ray-cast kernels derive the samples per ray themselves */
-    return launch_view_raycast(ctx, V, ray_launch(V, ctx->launch, candidate_rays(V)), nullptr, s);
+    const RayLaunch R = ray_launch(V, ctx->launch, candidate_rays(V), ctx->test_lanes);
+    ctx->renderer->lanes = R.lanes;
+    return launch_view_raycast(ctx, V, R, nullptr, s);
 }
 
 lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const RayLaunch& R,

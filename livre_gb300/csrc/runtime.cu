@@ -907,12 +907,37 @@ lv_status make_ray_view(lv_ctx* ctx, const lv_volume* vol, const lv_tf* tf,
     V.tf_last = float(tf->n - 1u);
     /* the finest voxel at the volume's centre (or a little off it for an eye
      * inside), then coarser levels as the LOD threshold allows */
-    const float dist = std::sqrt(eye[0] * eye[0] + eye[1] * eye[1] + eye[2] * eye[2]);
-    V.px_per_voxel = 0.5f * float(desc.height) * std::fabs(desc.camera.projection[5]) /
-                     (float(V.max_voxel_dim) * std::max(dist, 0.4f));
+    const float dist = std::max(
+        std::sqrt(eye[0] * eye[0] + eye[1] * eye[1] + eye[2] * eye[2]), 0.4f);
+    const float px_per_length =
+        0.5f * float(desc.height) * std::fabs(desc.camera.projection[5]);
+    V.px_per_voxel = px_per_length / (float(V.max_voxel_dim) * dist);
     for (uint32_t l = lod.min_lod; l + 1u < info.depth; ++l)
         if (2.0f * V.px_per_voxel <= lod.screen_space_error)
             V.px_per_voxel *= 2.0f;
+    /* the step follows from the finest level rendered (view_samples), which
+     * the LOD threshold gives at the volume's nearest point */
+    float samples = float(desc.samples_per_ray);
+    if (desc.samples_per_ray == 0)
+    {
+        float gap = 0.f;
+        for (int a = 0; a < 3; ++a)
+        {
+            const float d = std::max(std::max(V.gmin[a] - eye[a], eye[a] - V.gmax[a]), 0.0f);
+            gap += d * d;
+        }
+        float near_px = px_per_length / (float(V.max_voxel_dim) * std::max(std::sqrt(gap), 0.05f));
+        samples = float(V.max_voxel_dim);
+        for (uint32_t l = lod.min_lod; l + 1u < info.depth && 2.0f * near_px <= lod.screen_space_error;
+             ++l)
+        {
+            near_px *= 2.0f;
+            samples *= 0.5f;
+        }
+        samples = desc.step_policy == LV_STEP_HALF_VOXEL ? 2.0f * samples
+                                                         : std::max(samples, 512.0f);
+    }
+    V.px_per_step = px_per_length / (std::max(samples, 1.0f) * dist);
     V.accumulate = 0;
     V.max_base = V.edge ? 0u
                         : (V.N[2] - 2u) * V.N[1] * V.N[0] + (V.N[1] - 2u) * V.N[0] + V.N[0] - 2u;
@@ -1467,6 +1492,17 @@ extern "C" lv_status lv_get_render_launch(lv_ctx* ctx, lv_render_launch* cfg)
         return LV_EINVAL;
     std::lock_guard<std::mutex> lock(ctx->mutex);
     *cfg = ctx->launch;
+    return LV_OK;
+}
+
+extern "C" lv_status lv_test_ray_lanes(lv_ctx* ctx, uint32_t lanes, uint32_t* last)
+{
+    if (!ctx || (lanes != 0 && lanes != 1 && lanes != 4 && lanes != 8))
+        return fail(ctx, LV_EINVAL, "lanes per ray: 0 (by the rule), 1, 4 or 8");
+    std::lock_guard<std::mutex> lock(ctx->mutex);
+    ctx->test_lanes = lanes;
+    if (last)
+        *last = ctx->renderer ? ctx->renderer->lanes : 1u;
     return LV_OK;
 }
 
