@@ -127,6 +127,7 @@ struct RayView
     /* estimates for the host's choice of launch, at the volume's centre:
      * screen size of a rendered voxel's side and of a ray's step */
     float px_per_voxel, px_per_step;
+    float px_finest; /* the same of a voxel of the finest level */
     uint32_t samples_fixed; /* 0 = policy */
     uint32_t step_policy;
     uint32_t max_voxel_dim;

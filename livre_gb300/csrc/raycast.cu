@@ -1461,6 +1461,34 @@ lv_status refill_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch&
     return LV_OK;
 }
 
+/* Whether the one-lane tile kernel of V runs with 12 blocks an SM rather than
+ * 16 (raycast_tiles_roomy_kernel). uint16 taps are eight scattered loads a
+ * sample, so where neighbouring rays share few lines (the finest voxels are
+ * small on screen, whatever level is rendered) and the table takes its part of
+ * the L1, fewer rays at a time hit it more often; magnified voxels are shared
+ * and want the issue slots filled. The line by voxel size on screen rises with
+ * the table: 0.65 px at 256 entries, 1.3 at 4096 (fourth root); without a
+ * fixed pitch the roomy kernel needs 78 registers and pays up to 0.42 and 0.84
+ * px. Ray-cast ms with 16 / 12 blocks by (px_finest):
+ *   8192^3 in 128^3 bricks, 1080p, inside, 4096 entries  103.6 /  99.4 ( .16)
+ *     the same with 256 entries                           87.5 /  84.8 ( .16)
+ *   8192^3 in 128^3, orbit at 1.2, 4096 entries, 1080p     8.0 /   7.5 ( .08)
+ *   2048^3 in 64^3, orbit at 1.2, 256 entries, 1080p       6.9 /   6.5 ( .31)
+ *   1024^3 in 64^3, orbit at 1.2, 4096 entries, 2160p     11.0 /  10.6 (1.2)
+ *   2048^3 in 64^3, inside, 4096 entries, 2160p           31.1 /  32.5 (2.9)
+ *   1024^3 in 64^3, inside, 256 entries, 1440p             6.7 /   7.1 (3.8)
+ *   3072^3 in 96^3, orbit at 1.2, 4096 entries, 2160p     42.4 /  40.5 ( .41)
+ *     inside, LOD 2 px, 256 entries, 1080p                19.3 /  20.0 ( .44)
+ * Of 300 views none by this rule is over 3 % behind the better of the two, and
+ * 124 are 2 to 8 % ahead of 16 blocks. Bricks below 64^3 look up so often that
+ * 16 blocks are better or equal (512^3 in 32^3 bricks 1.54 / 1.67), as for
+ * uint8 (2048^3 in 64^3, orbit, 3.6 / 3.9) and the nearest filter. */
+bool roomy_l1(const RayView& V)
+{
+    const float line = fixed_pitch(V) ? 0.1625f : 0.105f;
+    return V.N[0] >= 64u && V.px_finest < line * std::sqrt(std::sqrt(V.tf_last + 1.0f));
+}
+
 /* One CTA per tile (LV_LAUNCH_TILE_GRID). */
 template <int DT, int F, int EDGE, int LA>
 lv_status tiles_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
@@ -1471,8 +1499,11 @@ lv_status tiles_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch& 
     if (st != LV_OK)
         return st;
     const uint32_t tiles = ((V.W + L.tile_w - 1) / L.tile_w) * ((V.H + L.tile_h - 1) / L.tile_h);
-    raycast_tiles_kernel<DT, F, EDGE, LA><<<tiles, L.tile_w * L.tile_h, 0, s>>>(V, L.tile_w,
-                                                                            L.tile_h, order);
+    auto k = raycast_tiles_kernel<DT, F, EDGE, LA>;
+    if constexpr (DT == LV_DT_UINT16 && F == LV_FILTER_TRILINEAR && EDGE != 1 && EDGE != 34 && LA)
+        if (roomy_l1(V))
+            k = raycast_tiles_roomy_kernel<DT, F, EDGE, LA>;
+    k<<<tiles, L.tile_w * L.tile_h, 0, s>>>(V, L.tile_w, L.tile_h, order);
     LV_CUDA(ctx, cudaGetLastError());
     return LV_OK;
 }
@@ -1521,38 +1552,27 @@ lv_status plain_dispatch_la(lv_ctx* ctx, const RayView& V, const lv_render_launc
     return LV_OK;
 }
 
-/* One CTA per tile for bricks of NX x NX voxels in x and y, the pitches as
- * immediates: 34, 66 and 130 are the 32^3, 64^3 and 128^3 bricks with an
- * overlap of 1. LA: one-sample look-ahead. */
-template <int DT, int F, int NX, int LA>
-lv_status tiles_nx_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
-                            cudaStream_t s, uint8_t* scratch)
-{
-    lv_status st = LV_OK;
-    const uint32_t* order = frame_order(ctx, V, L, scratch, s, st);
-    if (st != LV_OK)
-        return st;
-    const uint32_t tiles = ((V.W + L.tile_w - 1) / L.tile_w) * ((V.H + L.tile_h - 1) / L.tile_h);
-    raycast_tiles_kernel<DT, F, NX, LA><<<tiles, L.tile_w * L.tile_h, 0, s>>>(V, L.tile_w,
-                                                                            L.tile_h, order);
-    LV_CUDA(ctx, cudaGetLastError());
-    return LV_OK;
-}
-
 template <int DT, int F, int EDGE>
 lv_status plain_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
                          cudaStream_t s, uint8_t* scratch)
 {
-    if (EDGE == 0 && F == LV_FILTER_TRILINEAR && L.kind == LV_LAUNCH_TILE_GRID && fixed_pitch(V))
-    {
-        if (L.lookahead)
-            return V.N[0] == 66   ? tiles_nx_dispatch<DT, F, 66, 1>(ctx, V, L, s, scratch)
-                   : V.N[0] == 34 ? tiles_nx_dispatch<DT, F, 34, 1>(ctx, V, L, s, scratch)
-                                  : tiles_nx_dispatch<DT, F, 130, 1>(ctx, V, L, s, scratch);
-        return V.N[0] == 66   ? tiles_nx_dispatch<DT, F, 66, 0>(ctx, V, L, s, scratch)
-               : V.N[0] == 34 ? tiles_nx_dispatch<DT, F, 34, 0>(ctx, V, L, s, scratch)
-                              : tiles_nx_dispatch<DT, F, 130, 0>(ctx, V, L, s, scratch);
-    }
+    /* one CTA per tile for bricks of 34 x 34, 66 x 66 or 130 x 130 voxels in x
+     * and y (the 32^3, 64^3 and 128^3 bricks with an overlap of 1): the pitches
+     * as immediates */
+    if (EDGE == 0 && F == LV_FILTER_TRILINEAR && L.kind == LV_LAUNCH_TILE_GRID)
+        switch (fixed_pitch(V))
+        {
+        case 34:
+            return L.lookahead ? tiles_dispatch<DT, F, 34, 1>(ctx, V, L, s, scratch)
+                               : tiles_dispatch<DT, F, 34, 0>(ctx, V, L, s, scratch);
+        case 66:
+            return L.lookahead ? tiles_dispatch<DT, F, 66, 1>(ctx, V, L, s, scratch)
+                               : tiles_dispatch<DT, F, 66, 0>(ctx, V, L, s, scratch);
+        case 130:
+            return L.lookahead ? tiles_dispatch<DT, F, 130, 1>(ctx, V, L, s, scratch)
+                               : tiles_dispatch<DT, F, 130, 0>(ctx, V, L, s, scratch);
+        default: break;
+        }
     if (L.kind == LV_LAUNCH_WARP_REFILL)
         return refill_dispatch<DT, F, EDGE>(ctx, V, L, s);
     if (L.lookahead)

@@ -759,9 +759,8 @@ __device__ __forceinline__ bool skip_frame(const RayView& V)
 
 /* One CTA per tile: block i renders tile order[i] (or tile i). */
 template <int DT, int FILTER, int EDGE, int LA>
-__global__ void __launch_bounds__(256)
-    raycast_tiles_kernel(const RayView V, uint32_t tile_w, uint32_t tile_h,
-                         const uint32_t* __restrict__ order)
+__device__ __forceinline__ void cast_tile(const RayView& V, uint32_t tile_w, uint32_t tile_h,
+                                          const uint32_t* __restrict__ order)
 {
     if (skip_frame(V))
         return;
@@ -785,6 +784,25 @@ __global__ void __launch_bounds__(256)
         sum += __shfl_down_sync(0xFFFFFFFFu, sum, o);
     if ((threadIdx.x & 31u) == 0 && sum)
         atomicAdd(reinterpret_cast<unsigned long long*>(V.counters + FC_SAMPLES_LO), sum);
+}
+
+template <int DT, int FILTER, int EDGE, int LA>
+__global__ void __launch_bounds__(256)
+    raycast_tiles_kernel(const __grid_constant__ RayView V, uint32_t tile_w, uint32_t tile_h,
+                         const uint32_t* __restrict__ order)
+{
+    cast_tile<DT, FILTER, EDGE, LA>(V, tile_w, tile_h, order);
+}
+
+/* The same compiled for two resident blocks of 256 threads: 74 registers
+ * instead of 64 (uint16, trilinear, look-ahead), so 12 blocks of 64 threads
+ * share an SM's L1 instead of 16 (roomy_l1 chooses). */
+template <int DT, int FILTER, int EDGE, int LA>
+__global__ void __launch_bounds__(256, 2)
+    raycast_tiles_roomy_kernel(const __grid_constant__ RayView V, uint32_t tile_w,
+                               uint32_t tile_h, const uint32_t* __restrict__ order)
+{
+    cast_tile<DT, FILTER, EDGE, LA>(V, tile_w, tile_h, order);
 }
 
 /* ---------------------------------------------------------- split rays

@@ -911,7 +911,7 @@ lv_status make_ray_view(lv_ctx* ctx, const lv_volume* vol, const lv_tf* tf,
         std::sqrt(eye[0] * eye[0] + eye[1] * eye[1] + eye[2] * eye[2]), 0.4f);
     const float px_per_length =
         0.5f * float(desc.height) * std::fabs(desc.camera.projection[5]);
-    V.px_per_voxel = px_per_length / (float(V.max_voxel_dim) * dist);
+    V.px_finest = V.px_per_voxel = px_per_length / (float(V.max_voxel_dim) * dist);
     for (uint32_t l = lod.min_lod; l + 1u < info.depth; ++l)
         if (2.0f * V.px_per_voxel <= lod.screen_space_error)
             V.px_per_voxel *= 2.0f;
