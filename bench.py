@@ -86,6 +86,9 @@ def parse():
                         "stream), outofcore (8192^3 u16 fly-through through a 64 GiB pool), "
                         "outofcore_host (the same with host-generated bricks; not in the "
                         "default list: host generation takes tens of seconds per frame)")
+    p.add_argument("--details", default=None, metavar="FILE",
+                   help="writes the full record (every rate, configuration and note) as "
+                        "JSON; the printed line sums the modes up")
     p.add_argument("--cpu-frames", type=int, default=2,
                    help="whole frames the CPU baseline of the default line ray casts")
     p.add_argument("--serve-seconds", type=float, default=3.0,
@@ -1131,7 +1134,43 @@ def gb300_arm(args, cfg):
                                           "selection (1 thread) + FP64 ray cast of every row "
                                           "(%d threads), %.1f s per frame"
                                           % (ks, W, H, os.cpu_count(), sec)}
-    print(json.dumps(line), flush=True)
+    if args.details:
+        with open(args.details, "w") as f:
+            json.dump(line, f, indent=1)
+    print(json.dumps(compact(line)), flush=True)
+
+
+def compact(line):
+    """The line as printed, under 3 KB, so that a reader of the end of the
+    output has it whole: the headline's keys and, of each further mode, the
+    figures that sum it up, rounded. Notes and tables go to --details only."""
+    sums = {"served": ("capacity_served", "capacity_plain"),
+            "batched": ("plain", "batched", "persistent", "speedup_frames_per_s"),
+            "parity": ("tolerance", "max_err_255", "texture_filter_weights_max_err_255"),
+            "plain256": ("workload", "frames_per_s", "p50_ms", "raycast_ms_mean"),
+            "outofcore": ("workload", "frames_per_s", "raycast_ms_mean", "stream_ms_mean",
+                          "back_to_back_frames_per_s"),
+            "outofcore_host": ("frames_per_s",)}
+
+    def rounded(v):
+        if isinstance(v, float):
+            return float("%.6g" % v)
+        if isinstance(v, dict):
+            return {k: rounded(x) for k, x in v.items() if k not in ("note", "traffic_note")}
+        return v
+
+    out = {}
+    for key, value in line.items():
+        if key == "launch_sweep_raycast_ms":
+            continue
+        if key in sums:
+            value = {k: value[k] for k in sums[key] if k in value}
+            if key == "batched":
+                value = {k: v["frames_per_s"] if isinstance(v, dict) else v
+                         for k, v in value.items()}
+        # what the headline's consumers recompute stays as measured
+        out[key] = value if key in ("value", "ms_per_step") else rounded(value)
+    return out
 
 
 def main():
