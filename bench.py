@@ -1082,14 +1082,13 @@ def gb300_arm(args, cfg):
         "gpu_launches": int(sum(s["n_launches"] for s in stats)),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
-                     "traffic": None,
-                     "traffic_note": "not yet captured with the voxel-quad brick layout; the "
-                                     "last ncu capture of this launch (voxel pairs, 2 bytes "
-                                     "per voxel) read 37.11 MB and wrote 2.35 MB: the visible "
-                                     "bricks once, the 8-byte-per-sample gather served by "
-                                     "L1/L2",
+                     "traffic": TRAFFIC.get(args.config),
+                     "traffic_note": "dram__bytes_read + dram__bytes_write of one launch behind "
+                                     "an L2 flush (ncu): the 64 visible bricks' voxel quads "
+                                     "once; the 8-byte-per-sample gather is served by L1/L2",
                      "algorithmic_bytes_per_launch": float(alg_bytes.mean()),
-                     "kernel": "raycast_tiles_kernel<u8,trilinear>",
+                     "kernel": "lv_render's ray cast (raycast_split_kernel<u8,trilinear,66,4 "
+                               "lanes> in plain2048)",
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6800"},
         "e2e": {"value": replicas.job_rate(args.steps, world, e2e_total), "unit": "frames/s",
                 "h2d_bytes_per_step": int(h2d / args.steps),
@@ -1138,6 +1137,10 @@ def gb300_arm(args, cfg):
         with open(args.details, "w") as f:
             json.dump(line, f, indent=1)
     print(json.dumps(compact(line)), flush=True)
+
+
+# DRAM bytes of one ray-cast launch, by workload (ncu)
+TRAFFIC = {"plain2048": 73.6e6}
 
 
 def compact(line):
