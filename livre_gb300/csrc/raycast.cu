@@ -166,21 +166,22 @@ __device__ __forceinline__ void for_leaf_cells(const ResolveView& R, uint64_t id
 }
 
 /* Warps that share a node's cells where n nodes have nwarps warps: the fewer
- * nodes a frame renders, the more cells each covers. One warp for the 16.7 M
- * cells under the root of an 8192^3 octree in 32^3 bricks, shown small, made
- * a frame of 25.9 ms (asynchronous 38.6, with an atomic minimum per cell);
- * shared it is one of 86 us (93). The root of a 2048^3 octree in 64^3 bricks:
- * 122 -> 71 us. */
-__device__ __forceinline__ uint32_t cell_parts(uint32_t n, uint32_t nwarps)
+ * nodes a frame renders, the more cells each covers. At most one per 256 cells,
+ * so that a small grid is left to few warps. One warp for the 16.7 M cells
+ * under the root of an 8192^3 octree in 32^3 bricks, shown small, made a frame
+ * of 25.9 ms (asynchronous 38.6, with an atomic minimum per cell); shared it is
+ * one of 86 us (93). The root of a 2048^3 octree in 64^3 bricks: 122 -> 71 us. */
+__device__ __forceinline__ uint32_t cell_parts(const ResolveView& R, uint32_t n, uint32_t nwarps)
 {
-    return n && n < nwarps ? nwarps / n : 1u;
+    const uint32_t chunks = (R.dims[0] * R.dims[1] * R.dims[2]) >> 8;
+    return n && n < nwarps && n < chunks ? min(nwarps, chunks) / n : 1u;
 }
 
 /* Splats the rendering set into the leaf grid, a warp or several per entry. */
 __device__ void leaf_fill_body(const ResolveView& R, uint32_t warp, uint32_t nwarps)
 {
     const uint32_t n = min(R.counters[FC_RENDERED], R.render_capacity);
-    const uint32_t parts = cell_parts(n, nwarps);
+    const uint32_t parts = cell_parts(R, n, nwarps);
     for (uint32_t i = warp; i < n * parts; i += nwarps)
     {
         const uint32_t e = parts > 1u ? i % n : i;
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(256)
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n = *R.n_visible_ptr;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t parts = SYNC ? cell_parts(n, nwarps) : 1u;
+    const uint32_t parts = SYNC ? cell_parts(R, n, nwarps) : 1u;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n * parts; i += nwarps)
     {
         const uint32_t part = parts > 1u ? i / n : 0u;
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n = min(R.counters[FC_RENDERED], R.render_capacity);
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, parts = cell_parts(n, nwarps);
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, parts = cell_parts(R, n, nwarps);
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n * parts; i += nwarps)
     {
         const uint32_t part = parts > 1u ? i / n : 0u, e = i - part * n;
