@@ -124,10 +124,7 @@ struct RayView
                                a conservative bound of the pixels whose ray can
                                reach the volume's box; the others start and end
                                with no sample */
-    /* estimates for the host's choice of launch, at the volume's centre:
-     * screen size of a rendered voxel's side and of a ray's step */
-    float px_per_voxel, px_per_step;
-    float px_finest; /* the same of a voxel of the finest level */
+    float px_per_voxel;     /* estimated screen size of a rendered voxel's side */
     uint32_t samples_fixed; /* 0 = policy */
     uint32_t step_policy;
     uint32_t max_voxel_dim;
@@ -140,6 +137,9 @@ struct RayView
     uint32_t tfn;
     float4* out;
     uint32_t* counters; /* FrameCounters */
+    /* as px_per_voxel, of a ray's step and of a voxel of the finest level (the
+     * kernels read none of the three) */
+    float px_per_step, px_finest;
 };
 
 /* Device counters of one frame of one view. */

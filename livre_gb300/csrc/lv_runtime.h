@@ -215,6 +215,7 @@ lv_status run_selection(lv_ctx* ctx, const LodView* host_views,
                         uint32_t n_views, uint32_t max_depth,
                         cudaStream_t stream, bool allow_fused = true);
 
+using TileKernel = void (*)(RayView, uint32_t, uint32_t, const uint32_t*);
 /* The ray cast of a view as launched: its shape and the lanes that share a
  * ray (1, or 4 or 8 with one CTA per tile). */
 struct RayLaunch
@@ -344,6 +345,8 @@ struct Renderer
     cudaEvent_t t_sel0 = nullptr, t_sel1 = nullptr, t_ray0 = nullptr, t_ray1 = nullptr;
     uint32_t launches = 0;
     uint32_t lanes = 1; /* per ray, of the last frame's ray cast */
+    /* CTAs of a tile kernel that are resident at once, by block size */
+    std::map<std::pair<TileKernel, uint32_t>, uint32_t> resident_tiles;
     /* multi-pass frames: the visible set split into pool-sized passes */
     PinnedBuffer h_pass;     /* visible ids in pass order */
     DeviceBuffer pass_count; /* visible ids of the current pass */
@@ -416,19 +419,18 @@ void batch_set_priority_level(lv_batch* b, int level);
 /* Frame statistics from a view's counter words. */
 void batch_decode_stats(const uint32_t* words, lv_frame_stats& s);
 
-/* One view's ray cast as launch R, its longest-first tile order (if any) in `order_scratch` (tile_order_bytes; nullptr: the context's lv_render
- * scratch). The view's samples per ray must already be in its counters. */
+/* One view's ray cast as launch R, its longest-first tile order (if any) in
+ * `order_scratch` (tile_order_bytes; nullptr: the context's lv_render scratch,
+ * ordered ahead). The view's samples per ray must already be in its counters. */
 lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const RayLaunch& R,
                               uint8_t* order_scratch, cudaStream_t s);
 size_t tile_order_bytes(const RayView& V, const RayLaunch& R);
-/* The ray cast of a voxel type other than uint8 and uint16 (raycast_types.cu),
- * and of uint8 and uint16 with 4 or 8 lanes per ray (raycast_split.cu, `pitch`
- * the fixed pitch or 0): one CTA per tile of L, block i on tile order[i]
- * (null: tile i). */
-lv_status launch_other_type(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
-                            uint32_t lanes, const uint32_t* order, cudaStream_t s);
-lv_status launch_split(lv_ctx* ctx, const RayView& V, const lv_render_launch& L, uint32_t lanes,
-                       uint32_t pitch, const uint32_t* order, cudaStream_t s);
+/* A ray-cast kernel with one CTA per tile: (view, tile_w, tile_h, order), block
+ * i on tile order[i] (null: tile i). Those of the voxel types other than uint8
+ * and uint16 (raycast_types.cu; null: no such type), and of uint8 and uint16
+ * with 4 or 8 lanes per ray (raycast_split.cu, `pitch` the fixed pitch or 0). */
+TileKernel other_type_kernel(const RayView& V, const RayLaunch& R);
+TileKernel split_kernel(const RayView& V, uint32_t lanes, uint32_t pitch);
 /* Longest-first order of a batched group's work items (memset + 2 kernels);
  * hist: 128 words, keys and order: max_items entries (an upper bound of the
  * group's items at every replay of a captured launch). */

@@ -25,9 +25,9 @@
  * CPU oracle; shading runs in FP32 with fused multiply-adds.
  *
  * raycast_device.cuh holds the device code of a ray; this file the residency
- * and leaf-grid kernels, the launches of uint8 and uint16 volumes and the
- * dispatch; raycast_split.cu those with several lanes per ray and
- * raycast_types.cu the launches of the other voxel types.
+ * and leaf-grid kernels, the kernels of uint8 and uint16 volumes with one lane
+ * per ray and the dispatch; raycast_split.cu those with several lanes per ray
+ * and raycast_types.cu those of the other voxel types.
  */
 #include <algorithm>
 #include <cmath>
@@ -1410,18 +1410,100 @@ RayLaunch ray_launch(const RayView& V, const lv_render_launch& L, uint64_t rays,
     return R;
 }
 
+namespace
+{
+/* Whether the one-lane tile kernel of V runs with 12 blocks an SM rather than
+ * 16 (raycast_tiles_roomy_kernel). uint16 taps are eight scattered loads a
+ * sample, so where neighbouring rays share few lines (the finest voxels are
+ * small on screen, whatever level is rendered) and the table takes its part of
+ * the L1, fewer rays at a time hit it more often; magnified voxels are shared
+ * and want the issue slots filled. The line by voxel size on screen rises with
+ * the table: 0.65 px at 256 entries, 1.3 at 4096 (fourth root); without a
+ * fixed pitch the roomy kernel needs 78 registers and pays up to 0.42 and 0.84
+ * px. Ray-cast ms with 16 / 12 blocks by (px_finest):
+ *   8192^3 in 128^3 bricks, 1080p, inside, 4096 entries  103.6 /  99.4 ( .16)
+ *     the same with 256 entries                           87.5 /  84.8 ( .16)
+ *   8192^3 in 128^3, orbit at 1.2, 4096 entries, 1080p     8.0 /   7.5 ( .08)
+ *   2048^3 in 64^3, orbit at 1.2, 256 entries, 1080p       6.9 /   6.5 ( .31)
+ *   1024^3 in 64^3, orbit at 1.2, 4096 entries, 2160p     11.0 /  10.6 (1.2)
+ *   2048^3 in 64^3, inside, 4096 entries, 2160p           31.1 /  32.5 (2.9)
+ *   1024^3 in 64^3, inside, 256 entries, 1440p             6.7 /   7.1 (3.8)
+ *   3072^3 in 96^3, orbit at 1.2, 4096 entries, 2160p     42.4 /  40.5 ( .41)
+ *     inside, LOD 2 px, 256 entries, 1080p                19.3 /  20.0 ( .44)
+ * Of 300 views none by this rule is over 3 % behind the better of the two, and
+ * 124 are 2 to 8 % ahead of 16 blocks. Bricks below 64^3 look up so often that
+ * 16 blocks are better or equal (512^3 in 32^3 bricks 1.54 / 1.67), as for
+ * uint8 (2048^3 in 64^3, orbit, 3.6 / 3.9) and the nearest filter. */
+bool roomy_l1(const RayView& V)
+{
+    const float line = fixed_pitch(V) ? 0.1625f : 0.105f;
+    return V.N[0] >= 64u && V.px_finest < line * std::sqrt(std::sqrt(V.tf_last + 1.0f));
+}
+
+template <int DT, int F, int EDGE>
+TileKernel one_lane_kernel(const RayView& V, uint32_t lookahead)
+{
+    if constexpr (DT == LV_DT_UINT16 && F == LV_FILTER_TRILINEAR && EDGE != 1 && EDGE != 34)
+        if (lookahead && roomy_l1(V))
+            return raycast_tiles_roomy_kernel<DT, F, EDGE, 1>;
+    return lookahead ? raycast_tiles_kernel<DT, F, EDGE, 1> : raycast_tiles_kernel<DT, F, EDGE, 0>;
+}
+
+/* The kernels of bricks of 34 x 34, 66 x 66 and 130 x 130 voxels in x and y
+ * (the 32^3, 64^3 and 128^3 bricks with an overlap of 1) have the pitches as
+ * immediates. */
+template <int DT>
+TileKernel one_lane_kernel(const RayView& V, uint32_t lookahead)
+{
+    if (V.filter != LV_FILTER_TRILINEAR)
+        return V.edge ? one_lane_kernel<DT, LV_FILTER_NEAREST, 1>(V, lookahead)
+                      : one_lane_kernel<DT, LV_FILTER_NEAREST, 0>(V, lookahead);
+    switch (fixed_pitch(V))
+    {
+    case 34: return one_lane_kernel<DT, LV_FILTER_TRILINEAR, 34>(V, lookahead);
+    case 66: return one_lane_kernel<DT, LV_FILTER_TRILINEAR, 66>(V, lookahead);
+    case 130: return one_lane_kernel<DT, LV_FILTER_TRILINEAR, 130>(V, lookahead);
+    default:
+        return V.edge ? one_lane_kernel<DT, LV_FILTER_TRILINEAR, 1>(V, lookahead)
+                      : one_lane_kernel<DT, LV_FILTER_TRILINEAR, 0>(V, lookahead);
+    }
+}
+
+/* The kernel of V as launch R with one CTA per tile (null: unknown type). */
+TileKernel tile_kernel(const RayView& V, const RayLaunch& R)
+{
+    if (V.dtype != LV_DT_UINT8 && V.dtype != LV_DT_UINT16)
+        return other_type_kernel(V, R);
+    if (R.lanes > 1)
+        return split_kernel(V, R.lanes, fixed_pitch(V));
+    return V.dtype == LV_DT_UINT8 ? one_lane_kernel<LV_DT_UINT8>(V, R.shape.lookahead)
+                                  : one_lane_kernel<LV_DT_UINT16>(V, R.shape.lookahead);
+}
+
+uint32_t tiles_of(const RayView& V, const lv_render_launch& L)
+{
+    return ((V.W + L.tile_w - 1) / L.tile_w) * ((V.H + L.tile_h - 1) / L.tile_h);
+}
+} // namespace
+
 lv_status prepare_frame_order(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
                               cudaStream_t side, const uint32_t*& order)
 {
     order = nullptr;
-    const lv_render_launch T = ray_launch(V, L, candidate_rays(V), ctx->test_lanes).shape;
-    /* tiles that are all resident at once (64-thread blocks, 12 per SM at
-     * least) start together in any order: no order is computed, three launches
-     * fewer */
-    const uint64_t tiles = uint64_t((V.W + T.tile_w - 1) / T.tile_w) *
-                           ((V.H + T.tile_h - 1) / T.tile_h);
-    if (T.kind == LV_LAUNCH_TILE_GRID && T.tile_w * T.tile_h <= 64 && tiles <= 12u * 152u)
-        return LV_OK;
+    const RayLaunch R = ray_launch(V, L, candidate_rays(V), ctx->test_lanes);
+    const lv_render_launch& T = R.shape;
+    if (T.kind == LV_LAUNCH_TILE_GRID)
+    {
+        /* tiles that are all resident at once start together in any order: no
+         * order is computed, three launches fewer */
+        const uint32_t threads = T.tile_w * T.tile_h * R.lanes;
+        const TileKernel k = tile_kernel(V, R);
+        uint32_t& resident = ctx->renderer->resident_tiles[{k, threads}];
+        if (k && resident == 0)
+            resident = resident_ctas(ctx, k, int(threads), 0);
+        if (tiles_of(V, T) <= resident)
+            return LV_OK;
+    }
     if (T.kind == LV_LAUNCH_GRID || T.order != LV_ORDER_LONGEST_FIRST)
         return LV_OK;
     lv_status st = LV_OK;
@@ -1462,53 +1544,6 @@ lv_status refill_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch&
     return LV_OK;
 }
 
-/* Whether the one-lane tile kernel of V runs with 12 blocks an SM rather than
- * 16 (raycast_tiles_roomy_kernel). uint16 taps are eight scattered loads a
- * sample, so where neighbouring rays share few lines (the finest voxels are
- * small on screen, whatever level is rendered) and the table takes its part of
- * the L1, fewer rays at a time hit it more often; magnified voxels are shared
- * and want the issue slots filled. The line by voxel size on screen rises with
- * the table: 0.65 px at 256 entries, 1.3 at 4096 (fourth root); without a
- * fixed pitch the roomy kernel needs 78 registers and pays up to 0.42 and 0.84
- * px. Ray-cast ms with 16 / 12 blocks by (px_finest):
- *   8192^3 in 128^3 bricks, 1080p, inside, 4096 entries  103.6 /  99.4 ( .16)
- *     the same with 256 entries                           87.5 /  84.8 ( .16)
- *   8192^3 in 128^3, orbit at 1.2, 4096 entries, 1080p     8.0 /   7.5 ( .08)
- *   2048^3 in 64^3, orbit at 1.2, 256 entries, 1080p       6.9 /   6.5 ( .31)
- *   1024^3 in 64^3, orbit at 1.2, 4096 entries, 2160p     11.0 /  10.6 (1.2)
- *   2048^3 in 64^3, inside, 4096 entries, 2160p           31.1 /  32.5 (2.9)
- *   1024^3 in 64^3, inside, 256 entries, 1440p             6.7 /   7.1 (3.8)
- *   3072^3 in 96^3, orbit at 1.2, 4096 entries, 2160p     42.4 /  40.5 ( .41)
- *     inside, LOD 2 px, 256 entries, 1080p                19.3 /  20.0 ( .44)
- * Of 300 views none by this rule is over 3 % behind the better of the two, and
- * 124 are 2 to 8 % ahead of 16 blocks. Bricks below 64^3 look up so often that
- * 16 blocks are better or equal (512^3 in 32^3 bricks 1.54 / 1.67), as for
- * uint8 (2048^3 in 64^3, orbit, 3.6 / 3.9) and the nearest filter. */
-bool roomy_l1(const RayView& V)
-{
-    const float line = fixed_pitch(V) ? 0.1625f : 0.105f;
-    return V.N[0] >= 64u && V.px_finest < line * std::sqrt(std::sqrt(V.tf_last + 1.0f));
-}
-
-/* One CTA per tile (LV_LAUNCH_TILE_GRID). */
-template <int DT, int F, int EDGE, int LA>
-lv_status tiles_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
-                         cudaStream_t s, uint8_t* scratch)
-{
-    lv_status st = LV_OK;
-    const uint32_t* order = frame_order(ctx, V, L, scratch, s, st);
-    if (st != LV_OK)
-        return st;
-    const uint32_t tiles = ((V.W + L.tile_w - 1) / L.tile_w) * ((V.H + L.tile_h - 1) / L.tile_h);
-    auto k = raycast_tiles_kernel<DT, F, EDGE, LA>;
-    if constexpr (DT == LV_DT_UINT16 && F == LV_FILTER_TRILINEAR && EDGE != 1 && EDGE != 34 && LA)
-        if (roomy_l1(V))
-            k = raycast_tiles_roomy_kernel<DT, F, EDGE, LA>;
-    k<<<tiles, L.tile_w * L.tile_h, 0, s>>>(V, L.tile_w, L.tile_h, order);
-    LV_CUDA(ctx, cudaGetLastError());
-    return LV_OK;
-}
-
 template <int DT, int F, int EDGE, int LA>
 lv_status plain_dispatch_la(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
                             cudaStream_t s, uint8_t* scratch)
@@ -1528,8 +1563,6 @@ lv_status plain_dispatch_la(lv_ctx* ctx, const RayView& V, const lv_render_launc
         LV_CUDA(ctx, cudaGetLastError());
         return LV_OK;
     }
-    if (L.kind == LV_LAUNCH_TILE_GRID)
-        return tiles_dispatch<DT, F, EDGE, LA>(ctx, V, L, s, scratch);
     if (L.kind == LV_LAUNCH_TILE_QUEUE)
     {
         lv_status st = LV_OK;
@@ -1557,23 +1590,6 @@ template <int DT, int F, int EDGE>
 lv_status plain_dispatch(lv_ctx* ctx, const RayView& V, const lv_render_launch& L,
                          cudaStream_t s, uint8_t* scratch)
 {
-    /* one CTA per tile for bricks of 34 x 34, 66 x 66 or 130 x 130 voxels in x
-     * and y (the 32^3, 64^3 and 128^3 bricks with an overlap of 1): the pitches
-     * as immediates */
-    if (EDGE == 0 && F == LV_FILTER_TRILINEAR && L.kind == LV_LAUNCH_TILE_GRID)
-        switch (fixed_pitch(V))
-        {
-        case 34:
-            return L.lookahead ? tiles_dispatch<DT, F, 34, 1>(ctx, V, L, s, scratch)
-                               : tiles_dispatch<DT, F, 34, 0>(ctx, V, L, s, scratch);
-        case 66:
-            return L.lookahead ? tiles_dispatch<DT, F, 66, 1>(ctx, V, L, s, scratch)
-                               : tiles_dispatch<DT, F, 66, 0>(ctx, V, L, s, scratch);
-        case 130:
-            return L.lookahead ? tiles_dispatch<DT, F, 130, 1>(ctx, V, L, s, scratch)
-                               : tiles_dispatch<DT, F, 130, 0>(ctx, V, L, s, scratch);
-        default: break;
-        }
     if (L.kind == LV_LAUNCH_WARP_REFILL)
         return refill_dispatch<DT, F, EDGE>(ctx, V, L, s);
     if (L.lookahead)
@@ -1667,16 +1683,18 @@ lv_status launch_view_raycast(lv_ctx* ctx, const RayView& V, const RayLaunch& R,
 {
     const lv_render_launch& L = R.shape;
     ++ctx->kernels; /* whichever launch it is */
-    const bool other = V.dtype != LV_DT_UINT8 && V.dtype != LV_DT_UINT16;
-    if (other || R.lanes > 1)
+    if (L.kind == LV_LAUNCH_TILE_GRID)
     {
-        /* one CTA per tile */
         lv_status st = LV_OK;
         const uint32_t* order = frame_order(ctx, V, L, order_scratch, s, st);
         if (st != LV_OK)
             return st;
-        return other ? launch_other_type(ctx, V, L, R.lanes, order, s)
-                     : launch_split(ctx, V, L, R.lanes, fixed_pitch(V), order, s);
+        const TileKernel k = tile_kernel(V, R);
+        if (!k)
+            return fail(ctx, LV_EINVAL, "unknown voxel type");
+        k<<<tiles_of(V, L), L.tile_w * L.tile_h * R.lanes, 0, s>>>(V, L.tile_w, L.tile_h, order);
+        LV_CUDA(ctx, cudaGetLastError());
+        return LV_OK;
     }
     switch (kernel_variant(V.dtype, V.filter, V.edge))
     {

@@ -988,15 +988,10 @@ __global__ void __launch_bounds__(kSplitThreads)
 }
 
 template <int DT, int FILTER, int EDGE>
-lv_status split_launch(lv_ctx* ctx, const RayView& V, const lv_render_launch& L, uint32_t lanes,
-                       const uint32_t* order, cudaStream_t s)
+TileKernel split_kernel_of(uint32_t lanes)
 {
-    const uint32_t tiles = ((V.W + L.tile_w - 1) / L.tile_w) * ((V.H + L.tile_h - 1) / L.tile_h);
-    auto k = lanes == 4 ? raycast_split_kernel<DT, FILTER, EDGE, 4>
-                        : raycast_split_kernel<DT, FILTER, EDGE, 8>;
-    k<<<tiles, kSplitThreads, 0, s>>>(V, L.tile_w, L.tile_h, order);
-    LV_CUDA(ctx, cudaGetLastError());
-    return LV_OK;
+    return lanes == 4 ? raycast_split_kernel<DT, FILTER, EDGE, 4>
+                      : raycast_split_kernel<DT, FILTER, EDGE, 8>;
 }
 
 } // namespace

@@ -34,7 +34,7 @@ def test_launches_of_resident_frames(gpu_ctx):
     # more tiles than fit the GPU at once: their keys and their order
     assert go(1920, 1080) == SMALL + 2
     # more pixels to clear than go with the counters: a clear of their own
-    assert go(4096, 2160, radius=6.0) == SMALL + 2 + 1
+    assert go(4096, 2160, radius=3.0) == SMALL + 2 + 1
     vol.close()
     tf.close()
 
