@@ -151,7 +151,7 @@ lv_status lv_select_visible_host(lv_ctx* ctx, const lv_volume_info* vol,
  * polls (64 ns sleeps) instead of 2^22: the other CTAs give up, the launch
  * returns, and the selection reports LV_SEL_OVERFLOW = 2 (lv_select_visible)
  * or error_flags 4 (lv_render). Selections of octrees whose widest level
- * fits one CTA (<= 256 nodes) run on one CTA and are not affected. polls:
+ * fits one CTA (<= 1024 nodes) run on one CTA and are not affected. polls:
  * 1 .. 2^22. */
 lv_status lv_test_fail_grid_barrier(lv_ctx* ctx, uint32_t polls);
 
