@@ -1338,16 +1338,19 @@ bool splittable(const lv_render_launch& L)
  * The trilinear uint8 kernels have the fewest loads per sample, so they fill
  * the issue slots with the fewest rays; clamped taps have the longest chains.
  *
- * uint16 and int8: rays * px_per_step separates what gains from what loses.
- * Of 1008 uint16 frames (bricks of 16^3 to 128^3, tables of 256 and 4096
- * entries, orbits and paths inside, both step policies) none with a product
- * up to 250 000 is over 12 % slower with four lanes than with one, 6 over 3 %
- * (by limits on rays and px_per_voxel alone 56, the worst 23 %); 1024^3 uint16:
- * (240 000 rays, .65) 391 / 264, (373 000, .41) 805 / 623, (581 000, .51) 1141
- * / 1179, inside (173 000, .96) 361 / 283, (307 000, 1.3) 422 / 422, (480 000,
- * 1.6) 526 / 602; 256^3 int8 (147 000, .5) 223 / 180, (373 000, .8) 334 / 405.
- * Clamped uint16 2048^3: (373 000, .4) 1133 / 844, (949 000, .33) 4307 / 3742,
- * (949 000, .65) 2226 / 2558, (2.6 M, .6) 11388 / 14437. */
+ * uint16: rays * px_per_step separates what gains from what loses. Up to
+ * 250 000 four lanes pay (1024^3 in 64^3 bricks: 240 000 rays, .65: 391 / 264
+ * us; 373 000, .41: 805 / 623; inside 173 000, .96: 361 / 283), above 500 000
+ * they do not (581 000, 1.0: 428 / 502; inside 480 000, 1.6: 526 / 602; in 128^3
+ * bricks 581 000, 1.0, 4096 table entries: 479 / 583). Between the two it is the
+ * data: long rays through a clear volume gain (512^3, 362 000, .9: 1143 / 946),
+ * rays that end early lose (581 000, .5: 1089 / 1179), so the limits by voxel
+ * size decide there; bricks below 64^3 lose (256^3 in 32^3, 373 000, .8: 232 /
+ * 262; clear 311 / 344). Clamped taps depend on the data throughout (uint8 in
+ * quads, 512^3, 1.0 M rays: 3682 / 1994 through a clear volume, 982 / 1167
+ * where rays end early), but for voxels stored as one byte, whose taps share
+ * most lines: product above 600 000, 380^3 uint8 in 48^3 bricks 993 / 1131,
+ * 256^3 int8 911 / 1104. */
 uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
 {
     if (!splittable(L))
@@ -1370,7 +1373,9 @@ uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
     else if (V.edge)
     {
         eight = 100000.f;
-        four = std::min(2000000.f / p, 600000.f / step);
+        four = 2000000.f / p;
+        if (V.dtype == LV_DT_INT8 || (V.dtype == LV_DT_UINT8 && !V.quads))
+            four = std::min(four, 600000.f / step);
     }
     else if (V.dtype == LV_DT_UINT8)
     {
@@ -1380,9 +1385,9 @@ uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
     else
     {
         eight = V.dtype == LV_DT_UINT16 ? 16384.f : 32768.f;
-        four = V.dtype == LV_DT_UINT16 || V.dtype == LV_DT_INT8
-                   ? 250000.f / step
-                   : p < 1.4f ? 600000.f : (p < 1.9f ? 800000.f : 500000.f) / p;
+        four = p < 1.4f ? 600000.f : (p < 1.9f ? 800000.f : 500000.f) / p;
+        if (V.dtype == LV_DT_UINT16)
+            four = std::max(250000.f / step, V.N[0] >= 64u ? std::min(four, 500000.f / step) : 0.f);
     }
     return r <= eight ? 8 : r <= four ? 4 : 1;
 }
