@@ -137,9 +137,10 @@ struct RayView
     uint32_t tfn;
     float4* out;
     uint32_t* counters; /* FrameCounters */
-    /* as px_per_voxel, of a ray's step and of a voxel of the finest level (the
-     * kernels read none of the three) */
-    float px_per_step, px_finest;
+    /* as px_per_voxel, of a ray's step, of a voxel of the finest level and of a
+     * rendered voxel at the volume's nearest point (the kernels read none of
+     * the four) */
+    float px_per_step, px_finest, px_near;
 };
 
 /* Device counters of one frame of one view. */

@@ -1350,7 +1350,10 @@ bool splittable(const lv_render_launch& L)
  * quads, 512^3, 1.0 M rays: 3682 / 1994 through a clear volume, 982 / 1167
  * where rays end early), but for voxels stored as one byte, whose taps share
  * most lines: product above 600 000, 380^3 uint8 in 48^3 bricks 993 / 1131,
- * 256^3 int8 911 / 1104. */
+ * 256^3 int8 911 / 1104. The nearest filter's single load gains nothing where
+ * the near voxels are magnified (px_near): 512^3 uint16, 494 000 rays, 1.7: 457 /
+ * 580, 344 000, 1.45: 356 / 415; but 471 000, 1.3: 870 / 864, 328 000, 1.1: 426 /
+ * 374. */
 uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
 {
     if (!splittable(L))
@@ -1368,7 +1371,8 @@ uint32_t split_lanes(const RayView& V, const lv_render_launch& L, uint64_t rays)
     else if (V.filter != LV_FILTER_TRILINEAR)
     {
         eight = 32768.f;
-        four = p < 1.2f ? 500000.f : 90000.f;
+        four = p < 1.2f ? std::max(std::min(500000.f, 700000.f / (V.px_near * V.px_near)), 90000.f)
+                        : 90000.f;
     }
     else if (V.edge)
     {

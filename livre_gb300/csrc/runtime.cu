@@ -911,31 +911,37 @@ lv_status make_ray_view(lv_ctx* ctx, const lv_volume* vol, const lv_tf* tf,
         std::sqrt(eye[0] * eye[0] + eye[1] * eye[1] + eye[2] * eye[2]), 0.4f);
     const float px_per_length =
         0.5f * float(desc.height) * std::fabs(desc.camera.projection[5]);
-    V.px_finest = V.px_per_voxel = px_per_length / (float(V.max_voxel_dim) * dist);
-    for (uint32_t l = lod.min_lod; l + 1u < info.depth; ++l)
-        if (2.0f * V.px_per_voxel <= lod.screen_space_error)
-            V.px_per_voxel *= 2.0f;
+    /* screen size of a rendered voxel at distance d, and the level's number of
+     * voxels a side */
+    const auto rendered = [&](float d, float& voxels) {
+        voxels = float(V.max_voxel_dim);
+        float px = px_per_length / (voxels * d);
+        for (uint32_t l = lod.min_lod; l + 1u < info.depth && 2.0f * px <= lod.screen_space_error;
+             ++l)
+        {
+            px *= 2.0f;
+            voxels *= 0.5f;
+        }
+        return px;
+    };
+    float gap = 0.f, voxels = 0.f;
+    for (int a = 0; a < 3; ++a)
+    {
+        const float d = std::max(std::max(V.gmin[a] - eye[a], eye[a] - V.gmax[a]), 0.0f);
+        gap += d * d;
+    }
+    gap = std::sqrt(gap);
+    V.px_finest = px_per_length / (float(V.max_voxel_dim) * dist);
+    V.px_per_voxel = rendered(dist, voxels);
+    V.px_near = rendered(std::max(gap, 0.4f), voxels);
     /* the step follows from the finest level rendered (view_samples), which
      * the LOD threshold gives at the volume's nearest point */
     float samples = float(desc.samples_per_ray);
     if (desc.samples_per_ray == 0)
     {
-        float gap = 0.f;
-        for (int a = 0; a < 3; ++a)
-        {
-            const float d = std::max(std::max(V.gmin[a] - eye[a], eye[a] - V.gmax[a]), 0.0f);
-            gap += d * d;
-        }
-        float near_px = px_per_length / (float(V.max_voxel_dim) * std::max(std::sqrt(gap), 0.05f));
-        samples = float(V.max_voxel_dim);
-        for (uint32_t l = lod.min_lod; l + 1u < info.depth && 2.0f * near_px <= lod.screen_space_error;
-             ++l)
-        {
-            near_px *= 2.0f;
-            samples *= 0.5f;
-        }
-        samples = desc.step_policy == LV_STEP_HALF_VOXEL ? 2.0f * samples
-                                                         : std::max(samples, 512.0f);
+        rendered(std::max(gap, 0.05f), voxels);
+        samples = desc.step_policy == LV_STEP_HALF_VOXEL ? 2.0f * voxels
+                                                         : std::max(voxels, 512.0f);
     }
     V.px_per_step = px_per_length / (std::max(samples, 1.0f) * dist);
     V.accumulate = 0;
