@@ -1346,11 +1346,11 @@ bool splittable(const lv_render_launch& L)
  * data: long rays through a clear volume gain (512^3, 362 000, .9: 1143 / 946),
  * rays that end early lose (581 000, .5: 1089 / 1179), so the limits by voxel
  * size decide there; bricks below 64^3 lose (256^3 in 32^3, 373 000, .8: 232 /
- * 262; clear 311 / 344). Clamped taps depend on the data throughout (uint8 in
- * quads, 512^3, 1.0 M rays: 3682 / 1994 through a clear volume, 982 / 1167
- * where rays end early), but for voxels stored as one byte, whose taps share
- * most lines: product above 600 000, 380^3 uint8 in 48^3 bricks 993 / 1131,
- * 256^3 int8 911 / 1104. The nearest filter's single load gains nothing where
+ * 262; clear 311 / 344). Clamped taps depend on the data throughout (512^3,
+ * about 1 M rays: uint16 3682 / 1994 and uint8 in quads 3505 / 1958 through a
+ * clear volume, uint8 in quads 982 / 1167 where rays end early), but for voxels
+ * stored as one byte, whose taps share most lines: product above 600 000, 380^3
+ * uint8 in 48^3 bricks 993 / 1131, 256^3 int8 911 / 1104. The nearest filter's single load gains nothing where
  * the near voxels are magnified (px_near): 512^3 uint16, 494 000 rays, 1.7: 457 /
  * 580, 344 000, 1.45: 356 / 415; but 471 000, 1.3: 870 / 864, 328 000, 1.1: 426 /
  * 374. */
